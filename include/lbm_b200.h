@@ -182,9 +182,10 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks);
  * 22 = 20 with 3 stages. The ring variants are launched with programmatic stream
  * serialisation (the next step's blocks are scheduled while the previous step drains).
  * -1 (the default), by grid size from a sweep on GB300: rows narrower than 256 cells: 0; plain
- * FP32: 19 below 2^17 cells, 17 below 2^21, 12 above; 16-bit storage: 19 below 2^21 cells, 20
- * with rows of at least 2048 cells and 2^22 to 2^25 cells, 17 otherwise; FP64: 12 with at least
- * two 512-cell tiles per SM, 0 otherwise.
+ * FP32: 19 below 2^17 cells, 17 below 2^21, above a ring of its own (4 consumer warps, 2 passes,
+ * 2 stages, 5 blocks per SM; reported as 23); 16-bit storage: 19 below 2^21 cells, 20 with rows
+ * of at least 2048 cells and 2^22 to 2^25 cells, 17 otherwise; FP64: 12 or 19, whichever spreads
+ * its tiles more evenly over the SMs, 0 where a twentieth of the row's tiles lies past its end.
  * The 16-bit forms round stored populations stochastically (see lbm_create); every variant
  * derives the same random bits, so the variants give the same results. */
 int lbm_set_variant(lbm_solver* s, int variant);

@@ -307,17 +307,24 @@ struct BatchFlatPolicy {
     uint32_t mine = 0;
     if (lane < 3 * (S::WPS + 1)) mine = sm[(lane / (S::WPS + 1)) * S::MW + sd.w0 + lane % (S::WPS + 1)];
     const bool solids = __any_sync(0xffffffffu, mine != 0u);
+    if constexpr (S::LC == 2) {
 #pragma unroll 1
-    for (int c = 0; c < kC; ++c) {
-      const int x = sd.x0 + 32 * S::LC * c + S::LC * lane;
-      if (x < p.g.nx) {
-        const int lx = sd.lx0 + 32 * S::LC * c + S::LC * lane;
-        if constexpr (S::LC == 2)
-          ring_pair<ST, false, S, kRows>(p, st, sm, wr, sd.y, x, lx, sd.w0 + 2 * c, lane, solids, rkey);
-        else
-          ring_cell<ST, typename Phys::Arith, false, S, kRows>(p, st, sm, wr, sd.y, sd.ym, sd.yp, x, lx,
-                                                               sd.w0 + c, lane, solids);
+      for (int c = 0; c < kC; ++c) {
+        const int x = sd.x0 + 64 * c + 2 * lane;
+        if (x < p.g.nx)
+          ring_pair<ST, false, S, kRows>(p, st, sm, wr, sd.y, x, sd.lx0 + 64 * c + 2 * lane, sd.w0 + 2 * c, lane,
+                                         solids, rkey);
       }
+    } else {
+      with_force(p.k.force, [&](auto kind) {
+#pragma unroll 1
+        for (int c = 0; c < kC; ++c) {
+          const int x = sd.x0 + 32 * c + lane;
+          if (x < p.g.nx)
+            ring_cell<ST, typename Phys::Arith, decltype(kind)::value, false, S, kRows>(
+                p, st, sm, wr, sd.y, sd.ym, sd.yp, x, sd.lx0 + 32 * c + lane, sd.w0 + c, lane, solids);
+        }
+      });
     }
   }
 

@@ -10,6 +10,8 @@
 //   g_post = g - omega (g - g_eq) + (1 - omega/2) guo.
 #pragma once
 
+#include <cmath>
+
 #if defined(__CUDACC__)
 #define LBM_HD __host__ __device__ __forceinline__
 #else
@@ -43,7 +45,12 @@ struct CollideConsts {
   T hfx, hfy;         // real(0.5) * fx, real(0.5) * fy  (Guo half-force velocity shift)
   T cf_x, cf_y;       // c.F of directions 1 (= fx) and 2 (= fy)
   T cf_p, cf_q;       // c.F of directions 5 (fx + fy) and 6 ((-fx) + fy)
+  int force;          // which force components are non-zero (kForceNone / kForceX / kForceXY)
 };
+
+// Force kinds of the exact collision. Most flows are driven along x only, or by an inlet alone:
+// the Guo source then has fewer distinct terms (collide_exact_kind).
+constexpr int kForceNone = 0, kForceX = 1, kForceXY = 2;
 
 template <class T>
 inline CollideConsts<T> make_collide_consts(T tau, T fx, T fy) {
@@ -58,6 +65,7 @@ inline CollideConsts<T> make_collide_consts(T tau, T fx, T fy) {
   c.cf_y = fy;
   c.cf_p = fx + fy;
   c.cf_q = fy - fx;
+  c.force = fy != T(0) ? kForceXY : (fx != T(0) ? kForceX : kForceNone);
   return c;
 }
 
@@ -72,7 +80,13 @@ inline CollideConsts<T> make_collide_consts(T tau, T fx, T fy) {
 //   * opposite directions share values: RN(-a) = -RN(a), so cu_opp = -cu, 3 cu_opp = -(3 cu),
 //     (4.5 cu_opp) cu_opp = (4.5 cu) cu, (9 cu_opp) cf_opp = (9 cu) cf, and each such value is
 //     computed once;
-//   * (0 - u) f = -(u f) and a + (-b) = a - b are the same IEEE operation.
+//   * (0 - u) f = -(u f) and a + (-b) = a - b are the same IEEE operation;
+//   * products by powers of two are exact, so RN(4.5 a) = RN(9 a) / 2 and RN(RN(4.5 a) a) =
+//     RN(RN(9 a) a) / 2: the 9 a of the Guo source serves the equilibrium too, and the halving
+//     is folded into the following sum by an fma (a single rounding of an exact product plus the
+//     addend: the same sum). Likewise RN(4/9) = 4 RN(1/9) and RN(1/36) = RN(1/9) / 4. Where a
+//     underflows so far that a halving is inexact, the term is below half an ulp of 3 a;
+//   * a force component that is zero contributes zeros (collide_exact_kind).
 // Only the sign of an exact zero can differ from v0 (numerically equal: the reference's tests
 // compare with `!=`). A state holding inf or NaN has diverged; results then differ from v0 only
 // in which non-finite value they hold.
@@ -104,7 +118,10 @@ LBM_HD void moments_seq(const typename A::T (&g)[kQ], typename A::T& m0, typenam
 
 // Equilibrium, Guo source and BGK relaxation of one cell given its density, velocity and the
 // force acting on it (fx, fy; cf_p = fx + fy and cf_q = fy - fx, the c.F of directions 5 and 6).
-template <class A>
+// kForce: the force components that may be non-zero. With fy = 0 the products by fy are zeros:
+// t_0 = t_2 = t_4 = -(ux fx), t_1 = t_5 = t_8 = (1 - ux) fx, t_3 = t_6 = t_7 = (-1 - ux) fx,
+// P_2 = 0, c.F of directions 5 and 6 is fx and -fx; with no force the whole source is zero.
+template <class A, int kForce = kForceXY>
 LBM_HD void collide_exact_post(const typename A::T (&g)[kQ], typename A::T omega,
                                typename A::T force_prefactor, typename A::T drho, typename A::T rho,
                                typename A::T ux, typename A::T uy, typename A::T fx, typename A::T fy,
@@ -118,22 +135,21 @@ LBM_HD void collide_exact_post(const typename A::T (&g)[kQ], typename A::T omega
   const T a = ux, b = uy;
   const T p = A::add(ux, uy);
   const T q = A::sub(uy, ux);
-  const T three = A::k(S(3)), four5 = A::k(S(4.5)), nine = A::k(S(9));
+  const T three = A::k(S(3)), nine = A::k(S(9)), half = A::k(S(0.5));
   const T a3 = A::mul(three, a), b3 = A::mul(three, b), p3 = A::mul(three, p), q3 = A::mul(three, q);
-  const T ka = A::mul(A::mul(four5, a), a);
-  const T kb = A::mul(A::mul(four5, b), b);
-  const T kp = A::mul(A::mul(four5, p), p);
-  const T kq = A::mul(A::mul(four5, q), q);
+  const T a9 = A::mul(nine, a), b9 = A::mul(nine, b), p9 = A::mul(nine, p), q9 = A::mul(nine, q);
+  // Twice the 4.5 cu^2 terms.
+  const T ka = A::mul(a9, a), kb = A::mul(b9, b), kp = A::mul(p9, p), kq = A::mul(q9, q);
   // 3 cu + 4.5 cu^2 - 1.5 usq per direction (direction 0: -1.5 usq).
   T bracket[kQ];
-  bracket[1] = A::sub(A::add(a3, ka), s15);
-  bracket[3] = A::sub(A::sub(ka, a3), s15);
-  bracket[2] = A::sub(A::add(b3, kb), s15);
-  bracket[4] = A::sub(A::sub(kb, b3), s15);
-  bracket[5] = A::sub(A::add(p3, kp), s15);
-  bracket[7] = A::sub(A::sub(kp, p3), s15);
-  bracket[6] = A::sub(A::add(q3, kq), s15);
-  bracket[8] = A::sub(A::sub(kq, q3), s15);
+  bracket[1] = A::sub(A::fma(half, ka, a3), s15);
+  bracket[3] = A::sub(A::fma(half, ka, A::neg(a3)), s15);
+  bracket[2] = A::sub(A::fma(half, kb, b3), s15);
+  bracket[4] = A::sub(A::fma(half, kb, A::neg(b3)), s15);
+  bracket[5] = A::sub(A::fma(half, kp, p3), s15);
+  bracket[7] = A::sub(A::fma(half, kp, A::neg(p3)), s15);
+  bracket[6] = A::sub(A::fma(half, kq, q3), s15);
+  bracket[8] = A::sub(A::fma(half, kq, A::neg(q3)), s15);
 
   T geq[kQ];
   geq[0] = A::mul(A::k(weight<S>(0)), A::sub(drho, A::mul(rho, s15)));
@@ -142,58 +158,103 @@ LBM_HD void collide_exact_post(const typename A::T (&g)[kQ], typename A::T omega
 #endif
   for (int i = 1; i < kQ; ++i) geq[i] = A::mul(A::k(weight<S>(i)), A::add(drho, A::mul(rho, bracket[i])));
 
-  // Guo source: t_i = (cx_i - ux) fx + (cy_i - uy) fy from six products, P_i = (9 cu_i) cf_i.
-  const T axp = A::mul(A::sub(A::k(S(1)), ux), fx);
-  const T axm = A::mul(A::sub(A::k(S(-1)), ux), fx);
-  const T ax0 = A::neg(A::mul(ux, fx));
-  const T ayp = A::mul(A::sub(A::k(S(1)), uy), fy);
-  const T aym = A::mul(A::sub(A::k(S(-1)), uy), fy);
-  const T ay0 = A::neg(A::mul(uy, fy));
-  T t[kQ];
-  t[0] = A::add(ax0, ay0);
-  t[1] = A::add(axp, ay0);
-  t[2] = A::add(ax0, ayp);
-  t[3] = A::add(axm, ay0);
-  t[4] = A::add(ax0, aym);
-  t[5] = A::add(axp, ayp);
-  t[6] = A::add(axm, ayp);
-  t[7] = A::add(axm, aym);
-  t[8] = A::add(axp, aym);
-  const T pa = A::mul(A::mul(nine, a), fx);
-  const T pb = A::mul(A::mul(nine, b), fy);
-  const T pp = A::mul(A::mul(nine, p), cf_p);
-  const T pq = A::mul(A::mul(nine, q), cf_q);
-  T guo[kQ];
-  guo[0] = A::mul(A::k(weight<S>(0)), A::mul(three, t[0]));
-  guo[1] = A::mul(A::k(weight<S>(1)), A::add(A::mul(three, t[1]), pa));
-  guo[3] = A::mul(A::k(weight<S>(3)), A::add(A::mul(three, t[3]), pa));
-  guo[2] = A::mul(A::k(weight<S>(2)), A::add(A::mul(three, t[2]), pb));
-  guo[4] = A::mul(A::k(weight<S>(4)), A::add(A::mul(three, t[4]), pb));
-  guo[5] = A::mul(A::k(weight<S>(5)), A::add(A::mul(three, t[5]), pp));
-  guo[7] = A::mul(A::k(weight<S>(7)), A::add(A::mul(three, t[7]), pp));
-  guo[6] = A::mul(A::k(weight<S>(6)), A::add(A::mul(three, t[6]), pq));
-  guo[8] = A::mul(A::k(weight<S>(8)), A::add(A::mul(three, t[8]), pq));
-
+  // BGK part.
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-  for (int i = 0; i < kQ; ++i)
-    out[i] = A::add(A::sub(g[i], A::mul(omega, A::sub(g[i], geq[i]))), A::mul(force_prefactor, guo[i]));
+  for (int i = 0; i < kQ; ++i) out[i] = A::sub(g[i], A::mul(omega, A::sub(g[i], geq[i])));
+
+  // Guo source: t_i = (cx_i - ux) fx + (cy_i - uy) fy from six products, P_i = (9 cu_i) cf_i.
+  if (kForce == kForceX) {
+    const T w1 = A::k(weight<S>(1)), w5 = A::k(weight<S>(5));
+    const T z0 = A::mul(three, A::neg(A::mul(ux, fx)));
+    const T zp = A::mul(three, A::mul(A::sub(A::k(S(1)), ux), fx));
+    const T zm = A::mul(three, A::mul(A::sub(A::k(S(-1)), ux), fx));
+    const T pa = A::mul(a9, fx), pp = A::mul(p9, fx), nq = A::mul(q9, fx);  // P_6 = -nq
+    const T f2 = A::mul(force_prefactor, A::mul(w1, z0));  // directions 2 and 4; 0: 4 times
+    auto src = [&](T w, T z) { return A::mul(force_prefactor, A::mul(w, z)); };
+    out[0] = A::fma(A::k(S(4)), f2, out[0]);
+    out[1] = A::add(out[1], src(w1, A::add(zp, pa)));
+    out[3] = A::add(out[3], src(w1, A::add(zm, pa)));
+    out[2] = A::add(out[2], f2);
+    out[4] = A::add(out[4], f2);
+    out[5] = A::add(out[5], src(w5, A::add(zp, pp)));
+    out[7] = A::add(out[7], src(w5, A::add(zm, pp)));
+    out[6] = A::add(out[6], src(w5, A::sub(zm, nq)));
+    out[8] = A::add(out[8], src(w5, A::sub(zp, nq)));
+  } else if (kForce == kForceXY) {
+    const T axp = A::mul(A::sub(A::k(S(1)), ux), fx);
+    const T axm = A::mul(A::sub(A::k(S(-1)), ux), fx);
+    const T ax0 = A::neg(A::mul(ux, fx));
+    const T ayp = A::mul(A::sub(A::k(S(1)), uy), fy);
+    const T aym = A::mul(A::sub(A::k(S(-1)), uy), fy);
+    const T ay0 = A::neg(A::mul(uy, fy));
+    T t[kQ];
+    t[0] = A::add(ax0, ay0);
+    t[1] = A::add(axp, ay0);
+    t[2] = A::add(ax0, ayp);
+    t[3] = A::add(axm, ay0);
+    t[4] = A::add(ax0, aym);
+    t[5] = A::add(axp, ayp);
+    t[6] = A::add(axm, ayp);
+    t[7] = A::add(axm, aym);
+    t[8] = A::add(axp, aym);
+    const T pa = A::mul(a9, fx);
+    const T pb = A::mul(b9, fy);
+    const T pp = A::mul(p9, cf_p);
+    const T pq = A::mul(q9, cf_q);
+    T guo[kQ];
+    guo[0] = A::mul(A::k(weight<S>(0)), A::mul(three, t[0]));
+    guo[1] = A::mul(A::k(weight<S>(1)), A::add(A::mul(three, t[1]), pa));
+    guo[3] = A::mul(A::k(weight<S>(3)), A::add(A::mul(three, t[3]), pa));
+    guo[2] = A::mul(A::k(weight<S>(2)), A::add(A::mul(three, t[2]), pb));
+    guo[4] = A::mul(A::k(weight<S>(4)), A::add(A::mul(three, t[4]), pb));
+    guo[5] = A::mul(A::k(weight<S>(5)), A::add(A::mul(three, t[5]), pp));
+    guo[7] = A::mul(A::k(weight<S>(7)), A::add(A::mul(three, t[7]), pp));
+    guo[6] = A::mul(A::k(weight<S>(6)), A::add(A::mul(three, t[6]), pq));
+    guo[8] = A::mul(A::k(weight<S>(8)), A::add(A::mul(three, t[8]), pq));
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int i = 0; i < kQ; ++i) out[i] = A::add(out[i], A::mul(force_prefactor, guo[i]));
+  }
 }
 
-template <class A>
-LBM_HD void collide_exact(const typename A::T (&g)[kQ], const CollideConsts<typename A::T>& k,
-                          typename A::T (&out)[kQ]) {
+template <class A, int kForce>
+LBM_HD void collide_exact_kind(const typename A::T (&g)[kQ], const CollideConsts<typename A::T>& k,
+                               typename A::T (&out)[kQ]) {
   using T = typename A::T;
   using S = typename A::S;
   T m0, mx, my;
   moments_seq<A>(g, m0, mx, my);
   const T drho = m0;
   const T rho = A::add(A::k(S(1)), drho);
-  const T ux = A::div(A::add(mx, k.hfx), rho);
-  const T uy = A::div(A::add(my, k.hfy), rho);
-  collide_exact_post<A>(g, k.omega, k.force_prefactor, drho, rho, ux, uy, k.cf_x, k.cf_y, k.cf_p,
-                        k.cf_q, out);
+  const T ux = A::div(kForce == kForceNone ? mx : A::add(mx, k.hfx), rho);
+  const T uy = A::div(kForce == kForceXY ? A::add(my, k.hfy) : my, rho);
+  collide_exact_post<A, kForce>(g, k.omega, k.force_prefactor, drho, rho, ux, uy, k.cf_x, k.cf_y, k.cf_p,
+                                k.cf_q, out);
+}
+
+// Calls f(ForceKind<kind>) for a run-time force kind. The kind is the same for
+// every cell of a grid: the step kernels branch once per strip of cells, not per cell.
+template <int K>
+struct ForceKind {
+  static constexpr int value = K;
+};
+template <class F>
+LBM_HD void with_force(int force, F&& f) {
+  if (force == kForceX)
+    f(ForceKind<kForceX>{});
+  else if (force == kForceNone)
+    f(ForceKind<kForceNone>{});
+  else
+    f(ForceKind<kForceXY>{});
+}
+
+template <class A>
+LBM_HD void collide_exact(const typename A::T (&g)[kQ], const CollideConsts<typename A::T>& k,
+                          typename A::T (&out)[kQ]) {
+  with_force(k.force, [&](auto kind) { collide_exact_kind<A, decltype(kind)::value>(g, k, out); });
 }
 
 // The same collision with a Brinkman drag: the force on the cell is F_tot = F - alpha rho u and
@@ -376,6 +437,7 @@ struct HostArith {
   static inline T sub(T a, T b) { return a - b; }
   static inline T mul(T a, T b) { return a * b; }
   static inline T div(T a, T b) { return a / b; }
+  static inline T fma(T a, T b, T c) { return std::fma(a, b, c); }
 };
 
 }  // namespace lbm_b200

@@ -57,6 +57,13 @@ struct ExactF32 {
     return a * b;
 #endif
   }
+  static __host__ __device__ __forceinline__ float fma(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+    return __fmaf_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+  }
   static __host__ __device__ __forceinline__ float div(float a, float b) {
 #ifdef __CUDA_ARCH__
     return __fdiv_rn(a, b);
@@ -92,6 +99,13 @@ struct ExactF64 {
     return a * b;
 #endif
   }
+  static __host__ __device__ __forceinline__ double fma(double a, double b, double c) {
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+  }
   static __host__ __device__ __forceinline__ double div(double a, double b) {
 #ifdef __CUDA_ARCH__
     return __ddiv_rn(a, b);
@@ -119,6 +133,7 @@ struct ExactF32x2 {
   static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
   static __device__ __forceinline__ float2 sub(float2 a, float2 b) { return __fadd2_rn(a, neg(b)); }
   static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __ffma2_rn(a, b, kNegZero2); }
+  static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
   static __device__ __forceinline__ float2 div(float2 a, float2 b) {
     return make_float2(__fdiv_rn(a.x, b.x), __fdiv_rn(a.y, b.y));
   }

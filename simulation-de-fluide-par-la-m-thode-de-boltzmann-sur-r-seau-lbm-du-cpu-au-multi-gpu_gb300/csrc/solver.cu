@@ -187,9 +187,17 @@ int launch_async_t(lbm_solver* s, int steps) {
   return LBM_OK;
 }
 
+// Blocks per SM of the FP64 ring's grid. The collision is bound by the FP64 pipe, so what costs is
+// an uneven last wave: more blocks than reside (two or three) let the scheduler hand out the
+// last tiles one by one (1024 x 512: 2702 MLUPS with the resident grid, 3065 with 6 per SM).
+constexpr int kF64GridPerSm = 6;
+
 // Warp-specialised ring with one cell (plain FP32 / FP64) or one pair of cells (16-bit storage)
-// per lane (step_ring.cuh).
-template <class ST, bool kOpen, int kW, int kC, int kStages, int kMinBlocks>
+// per lane (step_ring.cuh). kMaxBlocks > 0 caps the resident blocks per SM (by the shared memory
+// a block asks for): past the bytes in flight that cover the latency, more of them only queue in
+// front of HBM and cost bandwidth (FP32, 4096^2, variant 12: 87.1k MLUPS at the 3 blocks per SM
+// it was tuned for, 78.5k at the 4 its 56 registers allow).
+template <class ST, bool kOpen, int kW, int kC, int kStages, int kMinBlocks, int kMaxBlocks = 0>
 int launch_ring_t(lbm_solver* s, int steps) {
   {
     using Phys = typename Form<ST>::Phys;
@@ -205,13 +213,16 @@ int launch_ring_t(lbm_solver* s, int steps) {
     const int tpr = (s->nx + S::TW - 1) / S::TW;
     const int tiles = tpr * s->ny;
     const auto kernel = ring_step_kernel<ST, Phys, kOpen, kW, kC, kStages, kMinBlocks>;
-    const size_t smem = ring_smem_bytes<S>(kStages);
+    size_t smem = ring_smem_bytes<S>(kStages);
+    if (kMaxBlocks > 0)  // 228 KB per SM, 1 KB of it reserved per block
+      smem = std::max<size_t>(smem, (228 * 1024 / std::max(kMaxBlocks, 1) - 1024) / 128 * 128);
     LBM_CUDA(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
     int grid = s->grid;
     if (grid <= 0) {
       int per_sm = 0;
       LBM_CUDA(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, S::kThreads, smem));
+      if (sizeof(ST) == 8) per_sm = kF64GridPerSm;
       grid = std::max(1, std::min(tiles, std::max(1, per_sm) * s->sm_count));
     }
     s->last_grid = grid;
@@ -231,6 +242,14 @@ int launch_ring_t(lbm_solver* s, int steps) {
   }
 }
 
+// Internal variant of the automatic choice: the ring with 4 consumer warps, 2 passes (256-cell
+// tiles), 2 stages and 5 resident blocks per SM, for plain FP32 on large grids. With fewer
+// instructions per cell the earlier choice (12, then 63 registers and so 3 blocks) drains its
+// stages faster and keeps too many bytes queued: 4096^2 MLUPS by shape and blocks per SM: 12
+// with 4 blocks 78.5k, 3 blocks 87.1k, 2 blocks 86.4k; 15 with 3 blocks 89.7k; this one with 4 / 5 / 6
+// blocks 89.0k / 90.9k / 79k (3000 x 5000: 87.9k / 91.1k / 79k; 2048^2: 85.4k / 87.8k / 84.6k).
+constexpr int kVariantF32Large = 23;
+
 // Automatic kernel choice (variant < 0), from a sweep of every variant on one GB300 (channel,
 // best of 3 runs, MLUPS): plain FP32: 256^2 v19 20.8k (v0 19.8k), 512^2 / 1024x256 v17 51.9k /
 // 51.7k (v12 47.4k / 46.2k), 1024^2 v17 83.9k (v12 81.7k), 2048^2 v12 86.2k, 4096^2 v12 90.6k;
@@ -242,23 +261,30 @@ int launch_ring_t(lbm_solver* s, int steps) {
 // v22 170.3k), 8192^2 v17 175.7k (v20 168.9k), so grids of at least 2^25 cells take v17.
 // Rows narrower than 256 cells take the
 // direct kernel (0), whose 128-cell chunks leave fewer lanes idle than the rings' wide tiles
-// (FP64 on 100 x 2000: the ring 12 reached 1.0k MLUPS with a fifth of its lanes busy); otherwise
-// FP64 (FP64-ALU-bound) takes the ring 12 with at least two of its tiles per SM, else 0.
+// (FP64 on 100 x 2000: the ring 12 reached 1.0k MLUPS with a fifth of its lanes busy). FP64 is
+// bound by the FP64 pipe: whole 256-cell tiles take the ring whose tile count (512 or 256 cells)
+// spreads more evenly over the SMs (1024 x 256: 12 2661 MLUPS, 19 3012; 2048^2: 3217 both), rows
+// whose 256-cell tiles are less than 95 % full the direct kernel (700 x 333: 19 2701, 0 3047).
 template <class ST>
 int auto_variant(const lbm_solver* s) {
   using S = RingShape<ST, 8, 2>;
   const long long cells = static_cast<long long>(s->nx) * s->ny;
   if (s->nx < 256) return 0;
   if (sizeof(ST) == 8) {
-    const long long tiles = static_cast<long long>((s->nx + S::TW - 1) / S::TW) * s->ny;
-    return tiles < 2LL * s->sm_count ? 0 : 12;
+    const int half = S::TW / 2;
+    if (20LL * s->nx < 19LL * ((s->nx + half - 1) / half * half)) return 0;
+    auto spread = [&](int tw) {  // busy share of the SMs over all waves of tiles
+      const double tiles = static_cast<double>((s->nx + tw - 1) / tw) * s->ny;
+      return tiles / (std::ceil(tiles / s->sm_count) * s->sm_count);
+    };
+    return spread(half) > 1.01 * spread(S::TW) ? 19 : 12;
   }
   if (sizeof(ST) == 2) {
     if (cells < (2LL << 20)) return 19;
     if (cells >= (32LL << 20)) return 17;
     return (s->nx >= 2048 && cells >= (4LL << 20)) ? 20 : 17;  // 2048-cell tiles need wide rows
   }
-  return cells < (1LL << 17) ? 19 : (cells < (2LL << 20) ? 17 : 12);
+  return cells < (1LL << 17) ? 19 : (cells < (2LL << 20) ? 17 : kVariantF32Large);
 }
 
 template <class ST, bool kOpen>
@@ -276,8 +302,8 @@ int launch_steps_o(lbm_solver* s, int steps) {
     case 9: return launch_async_t<ST, kOpen, 2>(s, steps);
     case 10: return launch_async_t<ST, kOpen, 3>(s, steps);
     case 11: return launch_async_t<ST, kOpen, 4>(s, steps);
-    case 12: return launch_ring_t<ST, kOpen, 8, 2, 2, 1>(s, steps);
-    case 13: return launch_ring_t<ST, kOpen, 8, 2, 3, 1>(s, steps);
+    case 12: return launch_ring_t<ST, kOpen, 8, 2, 2, 1, sizeof(ST) == 4 ? 3 : 0>(s, steps);
+    case 13: return launch_ring_t<ST, kOpen, 8, 2, 3, 1, sizeof(ST) == 4 ? 3 : 0>(s, steps);
     case 14: return launch_ring_t<ST, kOpen, 8, 2, 2, 4>(s, steps);
     case 15: return launch_ring_t<ST, kOpen, 4, 2, 3, 1>(s, steps);
     case 16: return launch_ring_t<ST, kOpen, 4, 2, 3, 7>(s, steps);
@@ -286,6 +312,7 @@ int launch_steps_o(lbm_solver* s, int steps) {
     case 19: return launch_ring_t<ST, kOpen, 8, 1, 4, 3>(s, steps);
     case 20: return launch_ring_t<ST, kOpen, 8, 4, 2, 2>(s, steps);
     case 21: return launch_ring_t<ST, kOpen, 4, 4, 2, 5>(s, steps);
+    case kVariantF32Large: return launch_ring_t<ST, kOpen, 4, 2, 2, 5, 5>(s, steps);
     case 22: return launch_ring_t<ST, kOpen, 8, 4, 3, 2>(s, steps);
     default: return launch_steps_t<ST, kOpen, 0>(s, steps);
   }

@@ -66,7 +66,8 @@ __device__ __forceinline__ int wrap_dir(int j) {
 // kWrapInRow: the stage holds the cell's whole row (columns 0 .. nx - 1 at lx - x ..), and the
 // periodic neighbours of x = 0 and x = nx - 1 are read from it instead of from wrap blocks.
 // kHalo: the strip engine's fused halo (StepArgs::halo_top / halo_bot).
-template <class ST, class A, bool kOpen, class S, bool kWrapInRow = false, bool kHalo = false>
+// kForce: the grid's force kind (CollideConsts::force).
+template <class ST, class A, int kForce, bool kOpen, class S, bool kWrapInRow = false, bool kHalo = false>
 __device__ __forceinline__ void ring_cell(const StepArgs<ST, ExactPhys<A>>& p, const ST* st,
                                           const uint32_t* sm, const ST* wr, int y, int ym, int yp,
                                           int x, int lx, int word, int lane, bool solids) {
@@ -137,7 +138,7 @@ __device__ __forceinline__ void ring_cell(const StepArgs<ST, ExactPhys<A>>& p, c
   (void)ym;
   (void)yp;
   T out[kQ];
-  collide_exact<A>(v, p.k, out);
+  collide_exact_kind<A, kForce>(v, p.k, out);
   ST* d = p.dst + static_cast<long long>(y) * p.g.pitch + x;
 #pragma unroll
   for (int i = 0; i < kQ; ++i) d[i * plane] = out[i];
@@ -362,17 +363,24 @@ __device__ __forceinline__ void ring_consume_tile(const StepArgs<ST, Phys>& p, c
   uint32_t mine = 0;
   if (lane < 3 * (S::WPS + 1)) mine = sm[(lane / (S::WPS + 1)) * S::MW + w0 + lane % (S::WPS + 1)];
   const bool solids = __any_sync(0xffffffffu, mine != 0u);
+  if constexpr (S::LC == 2) {
 #pragma unroll 1
-  for (int c = 0; c < kC; ++c) {
-    const int x = xw + 32 * S::LC * c + S::LC * lane;
-    if (x < nx) {
-      if constexpr (S::LC == 2)
+    for (int c = 0; c < kC; ++c) {
+      const int x = xw + 64 * c + 2 * lane;
+      if (x < nx)
         ring_pair<ST, kOpen, S, false, kHalo>(p, st, sm, wr, y, x, x - tx0 + S::H, w0 + 2 * c, lane, solids,
                                               step_rkey(p));
-      else
-        ring_cell<ST, typename Phys::Arith, kOpen, S, false, kHalo>(p, st, sm, wr, y, ym, yp, x, x - tx0 + S::H, w0 + c,
-                                                     lane, solids);
     }
+  } else {
+    with_force(p.k.force, [&](auto kind) {
+#pragma unroll 1
+      for (int c = 0; c < kC; ++c) {
+        const int x = xw + 32 * c + lane;
+        if (x < nx)
+          ring_cell<ST, typename Phys::Arith, decltype(kind)::value, kOpen, S, false, kHalo>(
+              p, st, sm, wr, y, ym, yp, x, x - tx0 + S::H, w0 + c, lane, solids);
+      }
+    });
   }
 }
 

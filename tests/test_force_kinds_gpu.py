@@ -1,0 +1,42 @@
+"""The exact collision's force kinds and the large-grid FP32 ring against the oracle (GPU): no
+force, force along x alone, along y alone and along both, on every kind of step kernel, equal
+value for value (the collision is bit-exact, so the tolerance is zero)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("real,prec", [("f32", "fp32"), ("f64", "fp64")])
+@pytest.mark.parametrize("force", [(0.0, 0.0), (1e-5, 0.0), (0.0, 1e-5), (1e-5, 2e-6)])
+@pytest.mark.parametrize("variant", [-1, 0, 7, 12, 19])
+def test_force_kinds(gpu_lib, orc, real, prec, force, variant):
+    nx, ny, steps = 259, 33, 12
+    mask = gpu_lib.geometry.add_block(gpu_lib.make_channel(nx, ny), nx, 30, 41, 9, 17)
+    dt = np.float32 if real == "f32" else np.float64
+    s0 = gpu_lib.workloads.seeded_state(5, 1e-2, nx, ny, mask, dt)
+    with gpu_lib.Solver(nx, ny, 0.7, *force, mask, precision=prec) as s:
+        s.set_variant(variant)
+        s.set_populations(s0)
+        s.run(steps)
+        got = s.populations()
+    want = orc.v0_run(nx, ny, mask, float(dt(0.7)), *force, s0, steps, real=real)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("nx,ny", [(2049, 1025), (8191, 257), (4096, 512)])
+def test_large_fp32_ring_equals_direct(gpu_lib, nx, ny):
+    """At least 2^21 cells: the automatic ring (256-cell tiles, ragged last tile) against the
+    direct kernel."""
+    mask = gpu_lib.geometry.add_block(gpu_lib.make_channel(nx, ny), nx, 250, 262, 90, 120)
+    s0 = gpu_lib.workloads.seeded_state(9, 1e-3, nx, ny, mask, np.float32)
+    got = []
+    for variant in (-1, 0):
+        with gpu_lib.Solver(nx, ny, 0.6, 1e-6, 0.0, mask) as s:
+            s.set_variant(variant)
+            s.set_populations(s0)
+            s.run(5)
+            got.append(s.populations())
+    assert np.array_equal(*got)
