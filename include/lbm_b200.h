@@ -114,7 +114,8 @@ int lbm_timed_run(lbm_solver* s, int steps, double* seconds);
 int lbm_synchronize(lbm_solver* s);
 
 /* Number of kernels s has enqueued for time steps so far: one per step plus one step-counter
- * update per launch sequence (a replayed step graph counts the kernels it holds). For
+ * update per launch sequence (a replayed step graph counts the kernels it holds, a launch that
+ * takes many steps counts one per step). For
  * benchmarks that report how many of the library's kernels ran in a timed region. */
 int lbm_kernel_launches(const lbm_solver* s, long long* count);
 
@@ -186,6 +187,9 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks);
  * 2 stages, 5 blocks per SM; reported as 23); 16-bit storage: 19 below 2^21 cells, 20 with rows
  * of at least 2048 cells and 2^22 to 2^25 cells, 17 otherwise; FP64: 12 or 19, whichever spreads
  * its tiles more evenly over the SMs, 0 where a twentieth of the row's tiles lies past its end.
+ * With -1 and no launch shape set, runs of at least 4 steps of an FP32 or 16-bit grid that fits the
+ * SMs' shared memory (up to about 370k cells in FP32, 750k with 16-bit storage, depending on the
+ * shape) keep the state there for the whole call, in one cooperative launch (reported as 24).
  * The 16-bit forms round stored populations stochastically (see lbm_create); every variant
  * derives the same random bits, so the variants give the same results. */
 int lbm_set_variant(lbm_solver* s, int variant);

@@ -20,6 +20,7 @@
 #include "solver_internal.h"
 #include "step_kernel.cuh"
 #include "step_async.cuh"
+#include "step_resident.cuh"
 #include "step_ring.cuh"
 #include "step_tma.cuh"
 #include "forms.cuh"
@@ -250,6 +251,17 @@ int launch_ring_t(lbm_solver* s, int steps) {
 // blocks 89.0k / 90.9k / 79k (3000 x 5000: 87.9k / 91.1k / 79k; 2048^2: 85.4k / 87.8k / 84.6k).
 constexpr int kVariantF32Large = 23;
 
+// Internal variant number of resident launches (step_resident.cuh). A launch loads and stores the
+// state and has no dependent-launch overlap, so short runs stay with the step kernels (us a step,
+// resident against them, runs of 2 / 3 / 4 / 16 / 400 steps: FP32 128 x 66 6.5 / 5.3 / 3.6 / 1.9 /
+// 1.4 against 6.5 / 5.2 / 4.7 / 3.5 / 3.0; 1024 x 256 8.5 / 7.4 / 5.6 / 3.3 / 2.5 against 8.4 / 7.5 /
+// 7.2 / 5.6 / 5.1; FP16 1021 x 700 11.2 / 10.4 / 7.6 / 4.9 / 4.0 against 11.1 / 9.9 / 10.0 / 8.7 /
+// 8.3; below four steps both columns are the step kernels): from four steps on every size that
+// fits is faster resident.
+constexpr int kVariantResident = 24;
+constexpr int kResidentMinSteps = 4;
+constexpr int kResidentSteps = 8192;  // steps per launch: a few tens of milliseconds
+
 // Automatic kernel choice (variant < 0), from a sweep of every variant on one GB300 (channel,
 // best of 3 runs, MLUPS): plain FP32: 256^2 v19 20.8k (v0 19.8k), 512^2 / 1024x256 v17 51.9k /
 // 51.7k (v12 47.4k / 46.2k), 1024^2 v17 83.9k (v12 81.7k), 2048^2 v12 86.2k, 4096^2 v12 90.6k;
@@ -318,8 +330,70 @@ int launch_steps_o(lbm_solver* s, int steps) {
   }
 }
 
+// Resident launches: the whole run of `steps` in cooperative launches of at most
+// kResidentSteps steps each, the state in the blocks' shared memory meanwhile.
+template <class ST, bool kOpen, int kForce>
+int launch_resident_t(lbm_solver* s, int steps) {
+  using Phys = typename Form<ST>::Phys;
+  using T = typename StoreTraits<ST>::T;
+  StepArgs<ST, Phys> a{};
+  a.mask = s->mask_d;
+  a.g = s->g;
+  a.k = Form<ST>::consts(s->tau, s->fx, s->fy);
+  const Eq9<T> e = step_inlet_eq<ST>(s);
+  for (int i = 0; i < kQ; ++i) a.eq_in[i] = e.v[i];
+  a.sc = s->sc;
+  a.dst = static_cast<ST*>(s->buf[s->cur]);
+  a.step_ctr = s->step_ctr;
+  const auto kernel = resident_step_kernel<ST, Phys, kOpen, kForce>;
+  LBM_CUDA(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(kResSmemBytes)));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(s->res.tx * s->res.ty);
+  cfg.blockDim = dim3(res_threads<ST>());
+  cfg.dynamicSmemBytes = kResSmemBytes;
+  cfg.stream = s->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  s->last_grid = s->res.tx * s->res.ty;
+  s->last_variant = kVariantResident;
+  while (steps > 0) {
+    const int n = std::min(steps, kResidentSteps);
+    LBM_CUDA(s, cudaLaunchKernelEx(&cfg, kernel, a, s->res, n, static_cast<LLWord*>(s->outbox), s->err_flag));
+    LBM_CUDA(s, launch_dependent(counter_add_dep_kernel, dim3(1), dim3(1), 0, s->stream, s->step_ctr,
+                                 static_cast<uint32_t>(n)));
+    steps -= n;
+  }
+  return LBM_OK;
+}
+
+template <class ST>
+int launch_resident(lbm_solver* s, int steps) {
+  if constexpr (sizeof(ST) == 4) {
+    int rc = LBM_OK;
+    with_force(Form<ST>::consts(s->tau, s->fx, s->fy).force, [&](auto kind) {
+      constexpr int K = decltype(kind)::value;
+      rc = s->open_x ? launch_resident_t<ST, true, K>(s, steps) : launch_resident_t<ST, false, K>(s, steps);
+    });
+    return rc;
+  } else {
+    return s->open_x ? launch_resident_t<ST, true, kForceXY>(s, steps) : launch_resident_t<ST, false, kForceXY>(s, steps);
+  }
+}
+
+// Runs of at least kResidentMinSteps steps take resident launches where the grid fits and the
+// caller has not chosen a kernel.
+bool use_resident(const lbm_solver* s, int steps) {
+  return s->res.tx > 0 && s->variant < 0 && s->grid == 0 && s->block == kStepThreads && steps >= kResidentMinSteps;
+}
+
 template <class ST>
 int launch_steps(lbm_solver* s, int steps) {
+  if constexpr (sizeof(ST) != 8)
+    if (use_resident(s, steps)) return launch_resident<ST>(s, steps);
   const int rc = s->open_x ? launch_steps_o<ST, true>(s, steps) : launch_steps_o<ST, false>(s, steps);
   if (rc) return rc;
   LBM_CUDA(s, launch_dependent(counter_add_dep_kernel, dim3(1), dim3(1), 0, s->stream, s->step_ctr,
@@ -436,6 +510,14 @@ int ensure_stage(lbm_solver* s, size_t bytes) {
   return LBM_OK;
 }
 
+// The cut of the grid for resident launches: tx = 0 where the grid does not fit.
+ResLayout plan_resident(const lbm_solver* s, bool open_x) {
+  if (s->elem == 4) return resident_layout<4>(s->nx, s->ny, s->sm_count, res_threads<float>() / 32, open_x);
+  if (s->elem == 2) return resident_layout<2>(s->nx, s->ny, s->sm_count, res_threads<__half>() / 32, open_x);
+  return ResLayout{};
+}
+size_t outbox_bytes(const ResLayout& L) { return 2 * static_cast<size_t>(L.words()) * L.tx * L.ty * sizeof(LLWord); }
+
 int check(const lbm_solver* s) { return s ? LBM_OK : LBM_ERR_INVALID_ARG; }
 
 // Storage scales: 1 for the plain forms, kStoreScale16 (2^15) on every plane of the 16-bit forms
@@ -503,7 +585,7 @@ int ensure_step_graph(lbm_solver* s) {
 // Steps: whole CUDA graphs of kGraphSteps launches for long runs on a non-default stream (no
 // per-launch host overhead, which dominates small grids), direct launches for the remainder.
 int solver_step_raw(lbm_solver* s, int steps) {
-  if (s->graphs && s->stream != nullptr && steps >= kGraphSteps) {
+  if (s->graphs && s->stream != nullptr && steps >= kGraphSteps && !use_resident(s, steps)) {
     if (int rc = ensure_step_graph(s)) return rc;
     while (s->graph && steps >= kGraphSteps) {
       LBM_CUDA(s, cudaGraphLaunch(s->graph, s->stream));
@@ -624,8 +706,25 @@ int lbm_create(int nx, int ny, const uint8_t* solid, double tau, double fx, doub
                         cudaMemcpyHostToDevice, s->stream);
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? LBM_ERR_OUT_OF_MEMORY : LBM_ERR_CUDA);
   s->red_blocks = 4 * s->sm_count;
-  e = cudaMalloc(&s->red, (s->red_blocks + 2) * sizeof(double) + 4 * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemsetAsync(s->red, 0, (s->red_blocks + 2) * sizeof(double) + 4 * sizeof(int), s->stream);
+  // One allocation: the reduction scratch, the flags, and from the next 256-byte boundary the
+  // outboxes of resident launches, for the closed cut and the open one.
+  const size_t red_bytes = (s->red_blocks + 2) * sizeof(double) + 4 * sizeof(int);
+  const size_t out_at = (red_bytes + 255) / 256 * 256;
+  int coop = 0, optin = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device);
+  size_t out_bytes = 0;
+  s->can_reside = coop && static_cast<size_t>(optin) >= kResSmemBytes;
+  if (s->can_reside) {
+    s->res = plan_resident(s, false);
+    out_bytes = std::max(outbox_bytes(s->res), outbox_bytes(plan_resident(s, true)));
+  }
+  e = cudaMalloc(&s->red, out_at + out_bytes);
+  if (e == cudaSuccess) e = cudaMemsetAsync(s->red, 0, red_bytes, s->stream);
+  if (e == cudaSuccess && out_bytes) {  // words tagged as no state's
+    s->outbox = reinterpret_cast<char*>(s->red) + out_at;
+    e = cudaMemsetAsync(s->outbox, 0xff, out_bytes, s->stream);
+  }
   s->err_flag = reinterpret_cast<int*>(s->red + s->red_blocks + 2) + 1;
   s->step_ctr = reinterpret_cast<uint32_t*>(s->red + s->red_blocks + 2) + 2;
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? LBM_ERR_OUT_OF_MEMORY : LBM_ERR_CUDA);
@@ -670,6 +769,7 @@ int lbm_set_inflow_outflow(lbm_solver* s, double u_in) {
   s->open_x = true;
   s->u_in = u_in;
   s->g.open_x = 1;
+  if (s->can_reside) s->res = plan_resident(s, true);
   lbm_b200::drop_step_graph(s);
   return LBM_OK;
 }

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "lbm_device.cuh"
+#include "resident_layout.h"
 
 struct lbm_solver {
   int nx = 0, ny = 0, precision = 0;
@@ -33,7 +34,7 @@ struct lbm_solver {
   double u_in = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  double* red = nullptr;  // mass partials [red_blocks], result, spare, then an int flag
+  double* red = nullptr;  // mass partials [red_blocks], result, spare, then int flags, then outboxes
   int red_blocks = 0;
   void* stage = nullptr;  // device staging for host input / output
   size_t stage_bytes = 0;
@@ -41,6 +42,11 @@ struct lbm_solver {
   int* err_flag = nullptr;  // set by a step kernel whose bounded wait ran out
   int variant = -1;      // step kernel variant (lbm_set_variant); -1: chosen from the grid shape
   int last_variant = 0;  // variant of the last launch
+  // Resident launches (step_resident.cuh): the device can run them, the cut of the grid (tx = 0:
+  // it does not fit), the tiles' outboxes (in red's allocation).
+  bool can_reside = false;
+  lbm_b200::ResLayout res{};
+  void* outbox = nullptr;
   int device = 0, sm_count = 0;
   lbm_b200::PlaneScales sc{};
   std::string err;
