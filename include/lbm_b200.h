@@ -254,7 +254,9 @@ int lbm_adj_get_tiles(const lbm_adjoint* a, int* forward_cells, int* backward_ce
 /* ---------------------------------------------------------------------------------------------
  * Batched ensemble (no counterpart in the reference): `count` independent closed channels of
  * uneven sizes, each with its own mask, tau and force, stepped together by one persistent kernel
- * launch per time step, replayed from a CUDA graph. Same arithmetic as the single-grid solver
+ * launch per time step, replayed from a CUDA graph; an FP32 or 16-bit ensemble of at most one
+ * instance per SM that fits the SMs' shared memory keeps its state there for a whole run while no
+ * launch shape has been set. Same arithmetic as the single-grid solver
  * (FP32 / FP64 bit-exact with the reference's v0 per instance).
  * ------------------------------------------------------------------------------------------- */
 typedef struct lbm_batch lbm_batch;

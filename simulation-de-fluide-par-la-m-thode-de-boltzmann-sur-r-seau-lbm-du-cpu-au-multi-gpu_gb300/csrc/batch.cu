@@ -32,6 +32,7 @@
 #include "forms.cuh"
 #include "fastdiv.h"
 #include "step_kernel.cuh"
+#include "step_resident.cuh"
 #include "step_ring.cuh"
 
 using namespace lbm_b200;
@@ -101,7 +102,8 @@ struct BatchArgs {
   int count;
   int items;
   PlaneScales sc;
-  const uint32_t* step;  // lattice steps taken (device counter; stochastic-rounding key)
+  const uint32_t* step;  // lattice steps taken before this launch sequence (device counter)
+  uint32_t step_off;     // index of this launch in the sequence (with it: the rounding key)
   const StagedArgs<ST, Phys>* args;  // [instance][parity]
   int parity;                        // src == buffer `parity`; odd parity walks the tiles backwards
   int tiles;                         // ring tiles of the ensemble
@@ -109,12 +111,18 @@ struct BatchArgs {
   const CopyOp* ops;                 // the tiles' copies
 };
 
-// Device step counter of a batch: read by every step launch, advanced by one after it (inside a
-// captured graph as well, so every replay of the graph rounds with fresh keys). Behind a ring
-// step it is a dependent launch (it waits for the step to complete), as is the next step.
-__global__ void step_counter_add(uint32_t* c) {
+// Device step counter of a batch: read by every step launch, advanced by their number after a
+// sequence of them (inside a captured graph as well, so every replay of the graph rounds with
+// fresh keys). Behind a step it is a dependent launch (it waits for the step to complete).
+__global__ void step_counter_add(uint32_t* c, uint32_t n) {
   grid_dependency_wait();
-  *c += 1u;
+  *c += n;
+}
+// The same after a resident launch, which also numbers its states (c[2]).
+__global__ void resident_counter_add(uint32_t* c, uint32_t n) {
+  grid_dependency_wait();
+  c[0] += n;
+  c[2] += n;
 }
 __global__ void step_counter_set(uint32_t* c, uint32_t v) { *c = v; }
 
@@ -147,7 +155,7 @@ __global__ void __launch_bounds__(kBatchThreads)
     p.k = d.k;
     p.sc = a.sc;
     p.step_ctr = a.step;
-    p.step_off = 0;
+    p.step_off = a.step_off;
     p.key_base = d.off / kQ;
     const Chunk c = chunk_at<G>(item - d.item0, d.cpr, d.g.nx, d.g.ny, lane);
     T v[kQ][G];
@@ -386,9 +394,37 @@ __global__ void __launch_bounds__(FlatShape<ST, kW, kC>::kThreads, (batch_ring_m
   using Pol = BatchFlatPolicy<ST, Phys, kW, kC>;
   extern __shared__ __align__(128) unsigned char smem[];
   grid_dependency_wait();
-  Pol pol{a, sizeof(ST) == 2 ? sr_step_key(__ldg(a.step)) : 0u};
+  Pol pol{a, sizeof(ST) == 2 ? sr_step_key(__ldg(a.step) + a.step_off) : 0u};
   tile_pipeline<kW, kStages, Pol::kStageBytes, FlatShape<ST, kW, kC>::kProd>(smem, pol, tiles, err);
 }
+
+// Resident launches of a small ensemble (step_resident.cuh): every instance is cut into tiles, and
+// block k of one cooperative launch has tile blocks[k].tile of instance blocks[k].inst.
+struct ResBlock {
+  int inst, tile;
+};
+struct ResInst {
+  ResLayout L;
+  long long out_off;  // the instance's outboxes, in words
+};
+template <class ST, class Phys, int kForce>
+__global__ void __launch_bounds__(res_threads<ST>(), 1)
+    batch_resident_kernel(const StagedArgs<ST, Phys>* args, int parity, const ResBlock* blocks, const ResInst* insts,
+                          int steps, LLWord* outboxes, const uint32_t* tag_ctr, int* err) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ StagedArgs<ST, Phys> s_args;
+  __shared__ ResInst s_inst;
+  const ResBlock b = blocks[blockIdx.x];
+  // The entry whose dst is the current buffer.
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(args + 2 * b.inst + (parity ^ 1));
+  for (int k = threadIdx.x; k < static_cast<int>(sizeof(s_args) / 4); k += blockDim.x)
+    reinterpret_cast<uint32_t*>(&s_args)[k] = src[k];
+  if (threadIdx.x == 0) s_inst = insts[b.inst];
+  __syncthreads();
+  resident_body<ST, Phys, false, kForce>(smem, s_args.p, s_inst.L, b.tile, steps, outboxes + s_inst.out_off, tag_ctr,
+                                         err);
+}
+static_assert(kResSmemBytes + 1024 <= 227 * 1024, "the resident block's arguments fit beside its buffers");
 
 template <class ST>
 struct BForm;
@@ -460,7 +496,15 @@ struct lbm_batch {
   cudaGraphExec_t graph = nullptr;
   int graph_cur = -1;  // buffer parity the graph was captured from
   uint32_t t = 0;             // lattice steps taken (host copy of *step_d)
-  uint32_t* step_d = nullptr;  // device: [0] step counter, [1] error flag of the bounded waits
+  // device: [0] step counter, [1] error flag of the bounded waits, [2] state number of resident
+  // launches (never put back)
+  uint32_t* step_d = nullptr;
+  // Resident launches: block table, instance cuts and outboxes in one allocation (null: the
+  // ensemble does not fit), used while the caller has chosen no launch shape.
+  char* res_d = nullptr;
+  int res_blocks = 0, res_force = kForceNone;
+  size_t res_inst_at = 0, res_out_at = 0;
+  bool chosen = false;
   int sm_count = 0, device = 0;
   std::string err, tune_report;
 };
@@ -709,11 +753,12 @@ int launch_batch_t(lbm_batch* b, int steps, bool prepare_only) {
   for (int s = 0; s < steps; ++s) {
     a.src = static_cast<const ST*>(b->buf[b->cur]);
     a.dst = static_cast<ST*>(b->buf[b->cur ^ 1]);
+    a.step_off = static_cast<uint32_t>(s);
     kernel<<<b->grid_eff, b->block, 0, b->stream>>>(a);
-    step_counter_add<<<1, 1, 0, b->stream>>>(b->step_d);
     ++b->t;
     b->cur ^= 1;
   }
+  step_counter_add<<<1, 1, 0, b->stream>>>(b->step_d, static_cast<uint32_t>(steps));
   const cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) return bfail(b, LBM_ERR_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
   return LBM_OK;
@@ -761,13 +806,14 @@ int launch_batch_ring_t(lbm_batch* b, int steps, bool prepare_only) {
     a.src = static_cast<const ST*>(b->buf[b->cur]);
     a.dst = static_cast<ST*>(b->buf[b->cur ^ 1]);
     a.parity = b->cur;
+    a.step_off = static_cast<uint32_t>(s);
     // Dependent launches (programmatic stream serialisation): the next launch is scheduled while
     // this one drains (+0.1-0.2 % on the benchmark ensemble).
     B_CUDA(b, launch_dependent(kernel, dim3(b->grid_eff), dim3(S::kThreads), smem, b->stream, a, b->tiles, err));
-    B_CUDA(b, launch_dependent(step_counter_add, dim3(1), dim3(1), 0, b->stream, b->step_d));
     ++b->t;
     b->cur ^= 1;
   }
+  B_CUDA(b, launch_dependent(step_counter_add, dim3(1), dim3(1), 0, b->stream, b->step_d, static_cast<uint32_t>(steps)));
   const cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) return bfail(b, LBM_ERR_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
   return LBM_OK;
@@ -809,8 +855,109 @@ int batch_steps(lbm_batch* b, int steps) {
   return batch_dispatch(b, steps, false);
 }
 
-// Runs `steps` steps: whole graphs of kGraphSteps launches, then the remainder directly.
+template <class ST, int kForce>
+int launch_resident_k(lbm_batch* b, int steps) {
+  using Phys = typename BForm<ST>::Phys;
+  if (!b->args_d) {  // the step arguments come with the table
+    if (b->table_sw == 0) {
+      b->table_sw = RingShape<ST, 8, 2>::SW;
+      b->table_kw = 8;
+    }
+    if (int rc = build_table<ST>(b, StoreTraits<ST>::kVec)) return rc;
+  }
+  const auto kernel = batch_resident_kernel<ST, Phys, kForce>;
+  B_CUDA(b, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResSmemBytes)));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(b->res_blocks);
+  cfg.blockDim = dim3(res_threads<ST>());
+  cfg.dynamicSmemBytes = kResSmemBytes;
+  cfg.stream = b->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  while (steps > 0) {
+    const int n = std::min(steps, kResidentSteps);
+    B_CUDA(b, cudaLaunchKernelEx(&cfg, kernel, static_cast<const StagedArgs<ST, Phys>*>(b->args_d), b->cur,
+                                 reinterpret_cast<const ResBlock*>(b->res_d),
+                                 reinterpret_cast<const ResInst*>(b->res_d + b->res_inst_at), n,
+                                 reinterpret_cast<LLWord*>(b->res_d + b->res_out_at),
+                                 static_cast<const uint32_t*>(b->step_d + 2), reinterpret_cast<int*>(b->step_d + 1)));
+    B_CUDA(b, launch_dependent(resident_counter_add, dim3(1), dim3(1), 0, b->stream, b->step_d,
+                               static_cast<uint32_t>(n)));
+    b->t += static_cast<uint32_t>(n);
+    steps -= n;
+  }
+  return LBM_OK;
+}
+
+int launch_resident(lbm_batch* b, int steps) {
+  switch (b->precision) {
+    case LBM_FP16_STORE: return launch_resident_k<__half, kForceXY>(b, steps);
+    case LBM_BF16_STORE: return launch_resident_k<__nv_bfloat16, kForceXY>(b, steps);
+    default: {
+      int rc = LBM_OK;
+      with_force(b->res_force, [&](auto kind) { rc = launch_resident_k<float, decltype(kind)::value>(b, steps); });
+      return rc;
+    }
+  }
+}
+
+// Cuts the ensemble for resident launches: the smallest number of items per tile for which all
+// instances' tiles are at most one per SM. Leaves res_d null where there is none.
+template <int kElem>
+int plan_resident(lbm_batch* b) {
+  int coop = 0, optin = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, b->device);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
+  if (!coop || static_cast<size_t>(optin) < kResSmemBytes + 1024 || b->count > b->sm_count ||
+      b->total_cells > static_cast<long long>(b->sm_count) * (kResPlaneBytes / kElem))
+    return LBM_OK;
+  std::vector<ResLayout> cut(b->count), best;
+  int lo = 1, hi = kResMaxItems;  // fewest items that fit, by bisection (fewer items, more tiles)
+  while (lo <= hi) {
+    const int items = (lo + hi) / 2;
+    long long tiles = 0;
+    for (int k = 0; k < b->count && tiles <= b->sm_count; ++k) {
+      cut[k] = resident_layout_for<kElem>(b->inst[k].nx, b->inst[k].ny, items);
+      tiles += cut[k].tx ? cut[k].tx * cut[k].ty : b->sm_count + 1;
+    }
+    if (tiles <= b->sm_count) {
+      best = cut;
+      hi = items - 1;
+    } else {
+      lo = items + 1;
+    }
+  }
+  if (best.empty()) return LBM_OK;
+  std::vector<ResBlock> blocks;
+  std::vector<ResInst> insts(b->count);
+  long long words = 0;
+  for (int k = 0; k < b->count; ++k) {
+    insts[k] = ResInst{best[k], words};
+    const int tiles = best[k].tx * best[k].ty;
+    for (int t = 0; t < tiles; ++t) blocks.push_back(ResBlock{k, t});
+    words += 2LL * best[k].words() * tiles;
+    const int force = b->inst[k].fy != 0 ? kForceXY : (b->inst[k].fx != 0 ? kForceX : kForceNone);
+    b->res_force = std::max(b->res_force, force);
+  }
+  auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+  b->res_inst_at = up(blocks.size() * sizeof(ResBlock));
+  b->res_out_at = b->res_inst_at + up(insts.size() * sizeof(ResInst));
+  const size_t out_bytes = static_cast<size_t>(words) * sizeof(LLWord);
+  B_CUDA(b, cudaMalloc(&b->res_d, b->res_out_at + out_bytes));
+  B_CUDA(b, cudaMemcpy(b->res_d, blocks.data(), blocks.size() * sizeof(ResBlock), cudaMemcpyHostToDevice));
+  B_CUDA(b, cudaMemcpy(b->res_d + b->res_inst_at, insts.data(), insts.size() * sizeof(ResInst), cudaMemcpyHostToDevice));
+  B_CUDA(b, cudaMemset(b->res_d + b->res_out_at, 0xff, out_bytes));  // words tagged as no state's
+  b->res_blocks = static_cast<int>(blocks.size());
+  return LBM_OK;
+}
+
+// Runs `steps` steps: a resident launch where the ensemble fits and the caller has chosen no
+// launch shape, else whole graphs of kGraphSteps launches, then the remainder directly.
 int batch_run(lbm_batch* b, int steps) {
+  if (b->res_d && !b->chosen && steps >= kResidentMinSteps) return launch_resident(b, steps);
   if (steps >= kGraphSteps && (b->graph == nullptr || b->graph_cur != b->cur)) {
     drop_graph(b);
     if (int rc = batch_dispatch(b, 0, true)) return rc;  // table and grid, outside the capture
@@ -871,7 +1018,7 @@ int separate_t(lbm_batch* b, int steps) {
       args[k].dst = dst + b->inst[k].off;
       kernel<<<grids[k], kStepThreads, 0, b->stream>>>(args[k]);
     }
-    step_counter_add<<<1, 1, 0, b->stream>>>(b->step_d);
+    step_counter_add<<<1, 1, 0, b->stream>>>(b->step_d, 1u);
     ++b->t;
     b->cur ^= 1;
   }
@@ -1004,9 +1151,9 @@ int time_steps(lbm_batch* b, int steps, double* seconds) {
 
 // Revision of the batch kernels in autotuner cache keys: raised whenever a change can reorder
 // the candidates or change what a cached launch means (2: two producer warps per ring block and
-// the resident-block caps that come with them; 3: the host-built copy plan), so that older
-// cached choices are timed again.
-constexpr int kBatchKernelRev = 3;
+// the resident-block caps that come with them; 3: the host-built copy plan; 4: the collision by
+// force kind and resident launches), so that older cached choices are timed again.
+constexpr int kBatchKernelRev = 4;
 
 std::string tune_key(const lbm_batch* b) {
   cudaDeviceProp prop{};
@@ -1102,6 +1249,8 @@ int lbm_batch_create(int count, const int* nx, const int* ny, const uint8_t* con
   if (e == cudaSuccess) e = cudaMalloc(&b->step_d, 4 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(b->step_d, 0, 4 * sizeof(uint32_t));
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? LBM_ERR_OUT_OF_MEMORY : LBM_ERR_CUDA);
+  if (elem != 8)
+    if (const int rc = elem == 4 ? plan_resident<4>(b) : plan_resident<2>(b)) return fail(rc);
   *out = b;
   return LBM_OK;
 }
@@ -1111,7 +1260,7 @@ int lbm_batch_destroy(lbm_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   drop_graph(b);
   for (void* p : {b->buf[0], b->buf[1], static_cast<void*>(b->mask_d), b->table_d, b->args_d, b->plans_d, b->ops_d, b->stage,
-                  static_cast<void*>(b->red), static_cast<void*>(b->step_d)})
+                  static_cast<void*>(b->red), static_cast<void*>(b->step_d), static_cast<void*>(b->res_d)})
     cudaFree(p);
   for (cudaEvent_t ev : b->ev)
     if (ev) cudaEventDestroy(ev);
@@ -1196,6 +1345,7 @@ int lbm_batch_set_launch(lbm_batch* b, int cells_per_thread, int block_threads, 
   b->G = cells_per_thread;
   b->block = block_threads;
   b->grid = grid_blocks;
+  b->chosen = true;
   drop_graph(b);
   return LBM_OK;
 }
@@ -1210,6 +1360,7 @@ int lbm_batch_set_tiles(lbm_batch* b, int consumer_warps, int passes, int stages
   b->ring_c = passes;
   b->ring_s = stages;
   b->G = 0;
+  b->chosen = true;
   drop_graph(b);
   return LBM_OK;
 }
@@ -1224,11 +1375,15 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
   auto apply = [&](const Cand& c) {
     if (c.G <= 1)
       if (int rc = lbm_batch_set_tiles(b, c.w, c.c, c.s)) return rc;
-    return lbm_batch_set_launch(b, c.G, c.blk, c.per_sm * b->sm_count);
+    if (int rc = lbm_batch_set_launch(b, c.G, c.blk, c.per_sm * b->sm_count)) return rc;
+    b->chosen = c.per_sm != 0;  // no blocks per SM: the resident launch
+    return static_cast<int>(LBM_OK);
   };
   auto describe = [&](const Cand& c) {
     std::ostringstream d;
-    if (c.G <= 1)
+    if (c.per_sm == 0)
+      d << "resident grid=" << b->res_blocks;
+    else if (c.G <= 1)
       d << "ring " << c.w << "x" << c.c << " stages=" << c.s << " grid=" << c.per_sm * b->sm_count;
     else
       d << "G=" << c.G << " block=" << c.blk << " grid=" << c.per_sm * b->sm_count;
@@ -1245,7 +1400,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
       if (std::getline(ls, k, '\t') && k == key && (ls >> G >> blk >> grd)) {
         ls >> w >> c >> s;
         const Cand cand{G, blk, grd / std::max(1, b->sm_count), w, c, s, 0.0};
-        if (apply(cand) == LBM_OK) {
+        if ((cand.per_sm != 0 || b->res_d) && apply(cand) == LBM_OK) {
           b->grid = grd;
           b->tune_report = "cached: " + describe(cand);
           if (report && report_size) std::snprintf(report, report_size, "%s", b->tune_report.c_str());
@@ -1258,6 +1413,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
   // is harmless for timing, and both are put back from a saved copy afterwards, on success and
   // on every error exit, together with the launch shape the ensemble had on entry.
   const uint32_t t_saved = b->t;
+  const bool entry_chosen = b->chosen;
   const int entry_G = b->G, entry_block = b->block, entry_grid = b->grid;
   const int entry_w = b->ring_w, entry_c = b->ring_c, entry_s = b->ring_s;
   const size_t bytes = static_cast<size_t>(b->total_elems) * b->elem + 256;
@@ -1278,6 +1434,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
       b->ring_w = entry_w;
       b->ring_c = entry_c;
       b->ring_s = entry_s;
+      b->chosen = entry_chosen;
       drop_graph(b);
     }
     return e1 != cudaSuccess ? e1 : e2;
@@ -1306,6 +1463,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
   if (H == V)
     for (int blk : {128, 256})
       for (int per_sm : {1, 2, 4, 8}) cands.push_back({V, blk, per_sm, 8, 2, 2, 0.0});
+  if (b->res_d) cands.push_back({0, kBatchThreads, 0, b->ring_w, b->ring_c, b->ring_s, 0.0});
   double best = 1e30;
   Cand pick = cands.front();
   std::ostringstream rep;
@@ -1315,7 +1473,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
     if (int rc = time_steps(b, 4, &t)) return fail_restored(rc);  // warm-up
     if (int rc = time_steps(b, 16, &t)) return fail_restored(rc);
     c.t = t;
-    rep << (c.G <= 1 ? "R" + std::to_string(c.w) + "x" + std::to_string(c.c) + "s" + std::to_string(c.s)
+    rep << (c.per_sm == 0 ? std::string("resident") : c.G <= 1 ? "R" + std::to_string(c.w) + "x" + std::to_string(c.c) + "s" + std::to_string(c.s)
                      : "G" + std::to_string(c.G) + "/b" + std::to_string(c.blk))
         << "/x" << c.per_sm << ":" << static_cast<long long>(b->total_cells * 16 / t / 1e6) << " ";
     if (t < best) {

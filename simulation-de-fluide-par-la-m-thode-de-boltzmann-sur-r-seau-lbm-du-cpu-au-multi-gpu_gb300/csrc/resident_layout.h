@@ -171,37 +171,77 @@ struct ResItems {
   }
 };
 
+// The cut into tx columns and ty bands, with tx = 0 where it is not one: columns are whole groups
+// wide (mask words, 128-byte lines), the outlet's column nx - 2 shares its tile, and a tile's
+// planes and tables fit the block.
+template <int kElem>
+inline ResLayout resident_cut(int nx, int ny, int tx, int ty, bool open_x) {
+  constexpr int GW = kElem == 2 ? 64 : 32;
+  ResLayout L;
+  int w = (nx + tx - 1) / tx;
+  if (tx > 1) w = (w + GW - 1) / GW * GW;
+  const int h = (ny + ty - 1) / ty;
+  if ((nx + w - 1) / w != tx || w > 4095 || h > 4095) return L;  // (fewer columns give the same cut)
+  if (open_x && nx - (tx - 1) * w < 2) return L;
+  if (static_cast<long long>(h + 2) * res_stride<kElem>(w) > kResPlaneBytes / kElem) return L;
+  if (ResItems<kElem>(w, h).total > kResMaxItems || (h + 2) * ((w + 2 + 31) / 32 + 1) > kResMaxMask ||
+      res_polls<kElem>(w, h) > kResMaxWords)
+    return L;
+  L.tx = tx;
+  L.ty = ty;
+  L.w = w;
+  L.base = ny / ty;
+  L.extra = ny % ty;
+  L.hs = h;
+  L.ws = res_row_words<kElem>(w);
+  return L;
+}
+// Items of a cut's largest tile.
+template <int kElem>
+inline int resident_items(const ResLayout& L) {
+  return ResItems<kElem>(L.w, L.hs).total;
+}
+
 // Cuts an nx x ny grid into at most `blocks` tiles for kElem-byte storage: the fewest rounds of
 // the block's `warps` warps over its items, then the fewest items, then the shortest edge.
 // Returns a layout with tx = 0 when no cut fits.
 template <int kElem>
 inline ResLayout resident_layout(int nx, int ny, int blocks, int warps, bool open_x) {
-  constexpr int GW = kElem == 2 ? 64 : 32;
-  constexpr int cap = kResPlaneBytes / kElem;
   ResLayout best;
   long long best_cost = -1;
   for (int tx = 1; tx <= blocks; ++tx) {
-    int w = (nx + tx - 1) / tx;
-    if (tx > 1) w = (w + GW - 1) / GW * GW;
-    const int cols = (nx + w - 1) / w;
-    if (cols != tx) continue;  // the same cut as with fewer columns
-    if (open_x && nx - (tx - 1) * w < 2) continue;  // the outlet reads column nx - 2
-    const int ty = std::min(ny, blocks / tx);
-    const int h = (ny + ty - 1) / ty;
-    const long long items = ResItems<kElem>(w, h).total;
-    if (items > kResMaxItems || static_cast<long long>(h + 2) * res_stride<kElem>(w) > cap) continue;
-    if ((h + 2) * ((w + 2 + 31) / 32 + 1) > kResMaxMask || res_polls<kElem>(w, h) > kResMaxWords) continue;
-    const long long rounds = (items + warps - 1) / warps;
-    const long long cost = (rounds * 1024 + items) * 65536 + res_polls<kElem>(w, h);
-    if (best_cost >= 0 && cost >= best_cost) continue;
-    best_cost = cost;
-    best.tx = tx;
-    best.ty = ty;
-    best.w = w;
-    best.base = ny / ty;
-    best.extra = ny % ty;
-    best.hs = h;
-    best.ws = res_row_words<kElem>(w);
+    const ResLayout L = resident_cut<kElem>(nx, ny, tx, std::min(ny, blocks / tx), open_x);
+    if (L.tx == 0) continue;
+    const long long items = resident_items<kElem>(L), rounds = (items + warps - 1) / warps;
+    const long long cost = (rounds * 1024 + items) * 65536 + res_polls<kElem>(L.w, L.hs);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = L;
+    }
+  }
+  return best;
+}
+
+// The closed cut of an nx x ny grid with the fewest tiles of at most `items` items each (tx = 0:
+// none), for ensembles that share the blocks.
+template <int kElem>
+inline ResLayout resident_layout_for(int nx, int ny, int items) {
+  ResLayout best;
+  const int max_tx = (nx + 31) / 32;
+  for (int tx = 1; tx <= max_tx; ++tx) {
+    // The tallest band that keeps the tile within `items` and the plane (both grow with it).
+    int lo = 0, hi = ny;
+    while (lo < hi) {
+      const int h = (lo + hi + 1) / 2, ty = (ny + h - 1) / h;
+      const ResLayout L = resident_cut<kElem>(nx, ny, tx, ty, false);
+      if (L.tx && resident_items<kElem>(L) <= items)
+        lo = h;
+      else
+        hi = h - 1;
+    }
+    if (lo == 0) continue;
+    const ResLayout L = resident_cut<kElem>(nx, ny, tx, (ny + lo - 1) / lo, false);
+    if (L.tx && (best.tx == 0 || L.tx * L.ty < best.tx * best.ty)) best = L;
   }
   return best;
 }

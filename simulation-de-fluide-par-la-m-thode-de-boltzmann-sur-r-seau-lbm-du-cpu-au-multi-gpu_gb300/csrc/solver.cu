@@ -259,8 +259,6 @@ constexpr int kVariantF32Large = 23;
 // 8.3; below four steps both columns are the step kernels): from four steps on every size that
 // fits is faster resident.
 constexpr int kVariantResident = 24;
-constexpr int kResidentMinSteps = 4;
-constexpr int kResidentSteps = 8192;  // steps per launch: a few tens of milliseconds
 
 // Automatic kernel choice (variant < 0), from a sweep of every variant on one GB300 (channel,
 // best of 3 runs, MLUPS): plain FP32: 256^2 v19 20.8k (v0 19.8k), 512^2 / 1024x256 v17 51.9k /

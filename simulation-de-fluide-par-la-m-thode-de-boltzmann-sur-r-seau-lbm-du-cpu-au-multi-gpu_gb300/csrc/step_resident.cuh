@@ -43,6 +43,9 @@
 namespace lbm_b200 {
 
 constexpr unsigned kResidentPolls = 1u << 22;  // about 2 s
+// Shortest run that takes a resident launch (solver.cu has the figures), and steps per launch (a
+// few tens of milliseconds).
+constexpr int kResidentMinSteps = 4, kResidentSteps = 8192;
 
 // One outbox word {v0, v1, v2, tag}: a 16-byte access that is single-copy atomic.
 struct alignas(16) LLWord {
@@ -225,14 +228,15 @@ __host__ __device__ constexpr int res_threads() {
   return sizeof(ST) == 2 ? 896 : 1024;
 }
 
-// The tile's steps. p.src is unused: the state is read from and written back to p.dst.
+// The steps of tile `tile` of the grid p, cut as L. The state is read from and written back to
+// p.dst (p.src is unused); `outboxes` are the grid's, of both parities; *tag_ctr numbers the states
+// (it only ever grows, see above), *p.step_ctr keys the stochastic rounding.
 template <class ST, class Phys, bool kOpen, int kForce>
-__global__ void __launch_bounds__(res_threads<ST>(), 1)
-    resident_step_kernel(const StepArgs<ST, Phys> p, const ResLayout L, int steps, LLWord* outboxes,
-                         int* err) {
+__device__ __forceinline__ void resident_body(unsigned char* smem, const StepArgs<ST, Phys>& p, const ResLayout& L,
+                                              int tile, int steps, LLWord* outboxes, const uint32_t* tag_ctr,
+                                              int* err) {
   constexpr int PS = kResPlaneBytes / static_cast<int>(sizeof(ST));
   constexpr int LC = sizeof(ST) == 2 ? 2 : 1, kThreads = res_threads<ST>();
-  extern __shared__ __align__(128) unsigned char smem[];
   ST* buf0 = reinterpret_cast<ST*>(smem);
   ST* buf1 = buf0 + 9 * PS;
   PollEntry* polls = reinterpret_cast<PollEntry*>(smem + 18 * static_cast<size_t>(kResPlaneBytes));
@@ -241,14 +245,14 @@ __global__ void __launch_bounds__(res_threads<ST>(), 1)
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nx = p.g.nx, ny = p.g.ny;
-  const int cy = static_cast<int>(blockIdx.x) / L.tx, cx = static_cast<int>(blockIdx.x) - cy * L.tx;
+  const int cy = tile / L.tx, cx = tile - cy * L.tx;
   const int w = L.width(cx, nx), h = L.height(cy), x0 = cx * L.w, y0 = L.row0(cy);
   const int rs = res_stride<static_cast<int>(sizeof(ST))>(w), c0 = res_col0<static_cast<int>(sizeof(ST))>();
   const ResItems<static_cast<int>(sizeof(ST))> items(w, h);
   const int nitems = items.total, npolls = res_polls<static_cast<int>(sizeof(ST))>(w, h);
   const int mw = (w + 2 + 31) / 32 + 1;
   const long long per_parity = static_cast<long long>(L.words()) * L.tx * L.ty;
-  const uint32_t t0 = __ldg(p.step_ctr);
+  const uint32_t t0 = __ldg(tag_ctr), step0 = sizeof(ST) == 2 ? __ldg(p.step_ctr) : 0u;
 
   // Tables: mask bits (bit j of a row: cell x0 - 1 + j; rows -1 .. h), poll list, items.
   for (int k = tid; k < (h + 2) * mw; k += kThreads) {
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(res_threads<ST>(), 1)
     }
   }
   __syncthreads();
-  LLWord* mine = outboxes + static_cast<long long>(blockIdx.x) * L.words();
+  LLWord* mine = outboxes + static_cast<long long>(tile) * L.words();
   {
     LLWord* ob = mine + (t0 & 1u) * per_parity;
     for (int e = warp; e < items.row_items + items.col_items; e += kThreads / 32) {
@@ -338,7 +342,7 @@ __global__ void __launch_bounds__(res_threads<ST>(), 1)
     const uint32_t tag = t0 + static_cast<uint32_t>(k) + 1u;
     const bool more = k + 1 < steps;
     LLWord* ob = mine + (tag & 1u) * per_parity;
-    const uint32_t rkey = sizeof(ST) == 2 ? sr_step_key(tag - 1u) : 0u;
+    const uint32_t rkey = sizeof(ST) == 2 ? sr_step_key(step0 + static_cast<uint32_t>(k)) : 0u;
     for (int e = warp; e < nitems; e += kThreads / 32) {
       const uint32_t it = table[e];
       int x = static_cast<int>(it & 0xfffu) + LC * lane, y = static_cast<int>((it >> 12) & 0xfffu);
@@ -370,6 +374,14 @@ __global__ void __launch_bounds__(res_threads<ST>(), 1)
         g[i * p.g.plane + static_cast<long long>(y) * p.g.pitch + x] = cur[i * PS + (y + 1) * rs + c0 + x];
     }
   }
+}
+
+// One grid: block k has tile k.
+template <class ST, class Phys, bool kOpen, int kForce>
+__global__ void __launch_bounds__(res_threads<ST>(), 1)
+    resident_step_kernel(const StepArgs<ST, Phys> p, const ResLayout L, int steps, LLWord* outboxes, int* err) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  resident_body<ST, Phys, kOpen, kForce>(smem, p, L, static_cast<int>(blockIdx.x), steps, outboxes, p.step_ctr, err);
 }
 
 }  // namespace lbm_b200

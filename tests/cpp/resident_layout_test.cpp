@@ -30,9 +30,8 @@ long fails = 0;
 using Slot = long long;
 
 template <int E>
-void grid(int nx, int ny, int blocks, bool open) {
+void grid(int nx, int ny, int blocks, bool open, const ResLayout& L) {
   constexpr int PS = kResPlaneBytes / E, LC = E == 2 ? 2 : 1;
-  const ResLayout L = resident_layout<E>(nx, ny, blocks, 28, open);
   if (L.tx == 0) return;
   CHECK(L.tx * L.ty <= blocks, "%dx%d: %d x %d tiles\n", nx, ny, L.tx, L.ty);
   const int tiles = L.tx * L.ty, nw = L.words(), c0 = res_col0<E>();
@@ -130,7 +129,13 @@ long sweep() {
       for (int nx : {1, 2, 3, 33, 64, 65, 66, 128, 300, 1021, 1025})
         for (int ny : {1, 2, 3, 7, 31, 152, 153, 320, 700}) {
           if (open && nx < 3) continue;
-          grid<E>(nx, ny, blocks, open);
+          grid<E>(nx, ny, blocks, open, resident_layout<E>(nx, ny, blocks, 28, open));
+          if (!open && blocks == 152) {
+            const int items = 5 + (nx * 7 + ny) % 60;
+            const ResLayout L = resident_layout_for<E>(nx, ny, items);
+            CHECK(L.tx == 0 || resident_items<E>(L) <= items, "%dx%d: more than %d items\n", nx, ny, items);
+            grid<E>(nx, ny, 1 << 20, false, L);
+          }
           ++n;
         }
     }

@@ -84,3 +84,35 @@ def test_two_resident_solvers_on_two_streams(gpu_lib):
             b.step(7)
         got = [a.populations(), b.populations()]
     assert np.array_equal(*got)
+
+
+def ensemble(pkg, count, lo, hi, fy):
+    specs = []
+    r = np.random.RandomState(count)
+    for k in range(count):
+        nx, ny = int(r.randint(lo, hi)), int(r.randint(3, hi // 2))
+        specs.append({"nx": nx, "ny": ny, "mask": channel(pkg, nx, ny), "tau": 0.55 + 0.4 * r.rand(),
+                      "fx": 1e-6 * k, "fy": fy})
+    return specs
+
+
+@pytest.mark.parametrize("count,lo,hi", [(1, 65, 66), (5, 3, 40), (24, 30, 200), (40, 64, 130), (152, 3, 33)])
+@pytest.mark.parametrize("form", ["fp32", "fp16", "bf16"])
+def test_resident_ensemble_equals_separate(gpu_lib, count, lo, hi, form):
+    """A small ensemble's resident launches against one launch per instance and step, with an
+    autotuning in between (it puts the step counter back: resident states keep their numbers)."""
+    specs = ensemble(gpu_lib, count, lo, hi, 3e-7 if count == 24 else 0.0)
+    got = []
+    for resident in (True, False):
+        with gpu_lib.Batch(specs, precision=form) as b:
+            b.init_equilibrium(1.0, 0.03, 0.01)
+            for n in (9, 4, 22):
+                if resident:
+                    b.run(n)
+                    if n == 9 and count == 5:
+                        b.autotune()
+                else:
+                    b.run_separate(n)
+            got.append([b.populations(k) for k in range(count)])
+    for a, c in zip(*got):
+        assert np.array_equal(a, c)
