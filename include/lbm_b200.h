@@ -185,8 +185,9 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks);
  * -1 (the default), by grid size from a sweep on GB300: rows narrower than 256 cells: 0; plain
  * FP32: 19 below 2^17 cells, 17 below 2^21, above a ring of its own (4 consumer warps, 2 passes,
  * 2 stages, 5 blocks per SM; reported as 23); 16-bit storage: 19 below 2^21 cells, 20 with rows
- * of at least 2048 cells and 2^22 to 2^25 cells, 17 otherwise; FP64: 12 or 19, whichever spreads
- * its tiles more evenly over the SMs, 0 where a twentieth of the row's tiles lies past its end.
+ * of at least 2048 cells and 2^22 to 2^25 cells, 17 otherwise; FP64: kernels of
+ * their own that multiply on the integer units, bit for bit the same (25: a ring, 26: the direct
+ * kernel, for rows below 256 cells or whose 256-cell tiles are less than 95 % full).
  * With -1 and no launch shape set, runs of at least 4 steps of an FP32 or 16-bit grid that fits the
  * SMs' shared memory (up to about 370k cells in FP32, 750k with 16-bit storage, depending on the
  * shape) keep the state there for the whole call, in one cooperative launch (reported as 24).

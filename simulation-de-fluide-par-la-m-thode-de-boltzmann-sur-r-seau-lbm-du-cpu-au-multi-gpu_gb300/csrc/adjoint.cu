@@ -293,6 +293,31 @@ __device__ __forceinline__ long long warp_slot(int b, int cw) {
 // Forward sweep
 // ---------------------------------------------------------------------------------------------
 
+// The drag collision of one cell; as collide_cell, a cell whose integer multiplications gave NaN
+// is collided again with the hardware's, out of line.
+template <class A>
+__device__ __noinline__ typename A::T collide_drag_rare(const typename A::T (&g)[kQ], CollideConsts<typename A::T> k,
+                                                        typename A::T alpha, typename A::T (&out)[kQ]) {
+  return collide_exact_drag<A>(g, k, alpha, out);
+}
+template <class A>
+__device__ __forceinline__ typename A::T collide_cell_drag(const typename A::T (&g)[kQ],
+                                                           const CollideConsts<typename A::T>& k,
+                                                           typename A::T alpha, typename A::T (&out)[kQ]) {
+  typename A::T ux = collide_exact_drag<A>(g, k, alpha, out);
+  if constexpr (std::is_same_v<A, ExactF64Int>) {
+    if (any_nan(out)) {
+      double v[kQ], o[kQ];
+#pragma unroll
+      for (int i = 0; i < kQ; ++i) v[i] = g[i];
+      ux = collide_drag_rare<ExactF64>(v, k, alpha, o);
+#pragma unroll
+      for (int i = 0; i < kQ; ++i) out[i] = o[i];
+    }
+  }
+  return ux;
+}
+
 template <class A, int kC>
 struct AdjForward {
   using T = typename A::T;
@@ -348,7 +373,7 @@ struct AdjForward {
     }
     const T alpha = p.alpha ? reinterpret_cast<const T*>(base + L::kAlpha)[lx - S::H] : T(0);
     T out[kQ];
-    const T ux = collide_exact_drag<A>(v, p.k, alpha, out);
+    const T ux = collide_cell_drag<A>(v, p.k, alpha, out);
     if (d) {
 #pragma unroll
       for (int i = 0; i < kQ; ++i) d[i * g.plane] = out[i];
@@ -656,11 +681,12 @@ __global__ void __launch_bounds__(kAuxThreads) slot_sum_kernel(const double* __r
 // Kernel configurations: cells per lane kC, ring depth and residency target. FP32: forward 3
 // stages at 3 blocks per SM (kC = 1: 32 KB, kC = 2: 63 KB of shared memory per block);
 // backward kC = 1 3 stages (64 KB) at 3 blocks per SM, kC = 2 2 stages (84 KB) at 2 blocks.
-// FP64 (kC = 1 only): forward 3 stages (63 KB), backward 2 stages (84 KB), 2 blocks per SM.
+// FP64 (kC = 1 only): forward 3 stages (63 KB) at 3 blocks per SM with integer multiplications,
+// backward 2 stages (84 KB), 2 blocks per SM.
 template <class T, int kC>
 struct AdjLaunch {
   static constexpr int kFwdStages = 3;
-  static constexpr int kFwdMin = sizeof(T) == 8 ? 2 : 3;
+  static constexpr int kFwdMin = 3;
   static constexpr int kBwdStages = (sizeof(T) == 8 || kC == 2) ? 2 : 3;
   static constexpr int kBwdMin = (sizeof(T) == 8 || kC == 2) ? 2 : 3;
   static constexpr size_t fwd_smem() { return adj_smem_bytes(FwdStage<T, kC>::kBytes, kFwdStages); }
@@ -1238,7 +1264,7 @@ int lbm_adj_create(int nx, int ny, const uint8_t* solid, double tau, double fx, 
       cudaEventCreateWithFlags(&a->join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&a->ev[0]) != cudaSuccess || cudaEventCreate(&a->ev[1]) != cudaSuccess)
     return fail(LBM_ERR_CUDA);
-  if (const int rc = precision == LBM_FP64 ? configure<ExactF64>(a) : configure<ExactF32>(a)) return fail(rc);
+  if (const int rc = precision == LBM_FP64 ? configure<ExactF64Int>(a) : configure<ExactF32>(a)) return fail(rc);
   std::vector<uint32_t> words;
   pack_mask(solid, nx, ny, a->g.mask_words, words);
   const size_t sb = state_bytes(a);
@@ -1292,7 +1318,7 @@ int lbm_adj_set_tiles(lbm_adjoint* a, int forward_cells, int backward_cells) {
     return adj_fail(a, LBM_ERR_INVALID_ARG, "cells per lane: 0 (automatic), 1, or 2 (FP32 only)");
   a->fwd_req = forward_cells;
   a->bwd_req = backward_cells;
-  return a->precision == LBM_FP64 ? configure<ExactF64>(a) : configure<ExactF32>(a);
+  return a->precision == LBM_FP64 ? configure<ExactF64Int>(a) : configure<ExactF32>(a);
 }
 
 int lbm_adj_get_tiles(const lbm_adjoint* a, int* forward_cells, int* backward_cells) {
@@ -1331,14 +1357,14 @@ int lbm_adj_set_alpha(lbm_adjoint* a, const double* alpha) {
 int lbm_adj_forward(lbm_adjoint* a, const void* s0, int steps, int window, double* J) {
   if (!a || !J || steps < 1 || window < 1 || window > steps + 1)
     return adj_fail(a, LBM_ERR_INVALID_ARG, "need steps >= 1 and 1 <= window <= steps + 1");
-  return a->precision == LBM_FP64 ? forward_t<ExactF64>(a, s0, steps, window, J)
+  return a->precision == LBM_FP64 ? forward_t<ExactF64Int>(a, s0, steps, window, J)
                                   : forward_t<ExactF32>(a, s0, steps, window, J);
 }
 
 int lbm_adj_backward(lbm_adjoint* a, double* dtau, double* dfx, double* dfy, double* dalpha) {
   if (!a) return LBM_ERR_INVALID_ARG;
   if (!a->have_forward) return adj_fail(a, LBM_ERR_INVALID_ARG, "run lbm_adj_forward first");
-  return a->precision == LBM_FP64 ? backward_t<ExactF64>(a, dtau, dfx, dfy, dalpha)
+  return a->precision == LBM_FP64 ? backward_t<ExactF64Int>(a, dtau, dfx, dfy, dalpha)
                                   : backward_t<ExactF32>(a, dtau, dfx, dfy, dalpha);
 }
 

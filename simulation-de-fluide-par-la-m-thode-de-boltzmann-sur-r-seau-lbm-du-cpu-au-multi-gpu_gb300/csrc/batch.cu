@@ -8,7 +8,7 @@
 // same chunk code as the single-grid kernel (step_kernel.cuh). The default kernel is instead the
 // warp-specialised ring of the single-grid solver (step_ring.cuh) over the ensemble's tiles of
 // consecutive row strips (a tile may cover several short rows): a tile's instance and place come
-// from a per-tile header built on the host (TileHead). Steps are replayed from a CUDA graph of
+// from a per-tile header built on the host (TilePlan). Steps are replayed from a CUDA graph of
 // kGraphSteps launches. lbm_batch_run_separate() runs the same instances one launch per
 // instance per step (the comparison point). lbm_batch_autotune() times the candidate launch
 // shapes (cells per thread G, i.e. the chunk width 32 G, threads per block, blocks per SM) on the
@@ -383,13 +383,15 @@ __host__ __device__ constexpr int batch_ring_blocks(int elem, int kW) {
 __host__ __device__ constexpr int batch_ring_tune_blocks(int elem, int kW) {
   return elem == 8 ? (kW == 8 ? 2 : (kW == 4 ? 4 : 6)) : batch_ring_blocks(elem, kW);
 }
-template <class ST, int kW>
+// FP64 with integer multiplications (the shape taken while none is chosen, 4 x 2 with 2 stages):
+// 4 blocks, 20 warps at 96 registers.
+template <class ST, class Phys, int kW>
 constexpr int batch_ring_min_blocks() {
-  return batch_ring_blocks(static_cast<int>(sizeof(ST)), kW);
+  return std::is_same_v<Phys, F64IntPhys> ? 4 : batch_ring_blocks(static_cast<int>(sizeof(ST)), kW);
 }
 
 template <class ST, class Phys, int kW, int kC, int kStages>
-__global__ void __launch_bounds__(FlatShape<ST, kW, kC>::kThreads, (batch_ring_min_blocks<ST, kW>()))
+__global__ void __launch_bounds__(FlatShape<ST, kW, kC>::kThreads, (batch_ring_min_blocks<ST, Phys, kW>()))
     batch_ring_kernel(const BatchArgs<ST, Phys> a, int tiles, int* err) {
   using Pol = BatchFlatPolicy<ST, Phys, kW, kC>;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -766,9 +768,8 @@ int launch_batch_t(lbm_batch* b, int steps, bool prepare_only) {
 
 // The ring kernel over the ensemble's tiles (one cell, or a pair with 16-bit storage, per lane),
 // tile shape kW consumer warps x kC passes, kStages ring stages per block.
-template <class ST, int kW, int kC, int kStages>
+template <class ST, int kW, int kC, int kStages, class Phys = typename BForm<ST>::Phys>
 int launch_batch_ring_t(lbm_batch* b, int steps, bool prepare_only) {
-  using Phys = typename BForm<ST>::Phys;
   using S = FlatShape<ST, kW, kC>;
   const auto kernel = batch_ring_kernel<ST, Phys, kW, kC, kStages>;
   const size_t smem = batch_ring_smem<BatchFlatPolicy<ST, Phys, kW, kC>>(kStages);
@@ -785,6 +786,7 @@ int launch_batch_ring_t(lbm_batch* b, int steps, bool prepare_only) {
     if (grid <= 0) {
       int per_sm = 0;
       B_CUDA(b, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, S::kThreads, smem));
+      if (std::is_same_v<Phys, F64IntPhys>) per_sm = kF64GridPerSm;
       grid = std::max(1, per_sm) * b->sm_count;
     }
     b->grid_eff = std::max(1, std::min(grid, b->tiles));
@@ -821,6 +823,8 @@ int launch_batch_ring_t(lbm_batch* b, int steps, bool prepare_only) {
 
 template <class ST>
 int launch_batch_ring(lbm_batch* b, int steps, bool prepare_only) {
+  if constexpr (sizeof(ST) == 8)
+    if (!b->chosen) return launch_batch_ring_t<ST, 4, 2, 2, F64IntPhys>(b, steps, prepare_only);
   const bool deep = b->ring_s == 4;
   if (b->ring_w == 4 && b->ring_c == 2)
     return deep ? launch_batch_ring_t<ST, 4, 2, 4>(b, steps, prepare_only) : launch_batch_ring_t<ST, 4, 2, 2>(b, steps, prepare_only);
@@ -1381,7 +1385,9 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
   };
   auto describe = [&](const Cand& c) {
     std::ostringstream d;
-    if (c.per_sm == 0)
+    if (c.per_sm == 0 && b->elem == 8)
+      d << "default";
+    else if (c.per_sm == 0)
       d << "resident grid=" << b->res_blocks;
     else if (c.G <= 1)
       d << "ring " << c.w << "x" << c.c << " stages=" << c.s << " grid=" << c.per_sm * b->sm_count;
@@ -1400,7 +1406,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
       if (std::getline(ls, k, '\t') && k == key && (ls >> G >> blk >> grd)) {
         ls >> w >> c >> s;
         const Cand cand{G, blk, grd / std::max(1, b->sm_count), w, c, s, 0.0};
-        if ((cand.per_sm != 0 || b->res_d) && apply(cand) == LBM_OK) {
+        if ((cand.per_sm != 0 || b->res_d || b->elem == 8) && apply(cand) == LBM_OK) {
           b->grid = grd;
           b->tune_report = "cached: " + describe(cand);
           if (report && report_size) std::snprintf(report, report_size, "%s", b->tune_report.c_str());
@@ -1463,7 +1469,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
   if (H == V)
     for (int blk : {128, 256})
       for (int per_sm : {1, 2, 4, 8}) cands.push_back({V, blk, per_sm, 8, 2, 2, 0.0});
-  if (b->res_d) cands.push_back({0, kBatchThreads, 0, b->ring_w, b->ring_c, b->ring_s, 0.0});
+  if (b->res_d || b->elem == 8) cands.push_back({0, kBatchThreads, 0, b->ring_w, b->ring_c, b->ring_s, 0.0});
   double best = 1e30;
   Cand pick = cands.front();
   std::ostringstream rep;
@@ -1473,7 +1479,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
     if (int rc = time_steps(b, 4, &t)) return fail_restored(rc);  // warm-up
     if (int rc = time_steps(b, 16, &t)) return fail_restored(rc);
     c.t = t;
-    rep << (c.per_sm == 0 ? std::string("resident") : c.G <= 1 ? "R" + std::to_string(c.w) + "x" + std::to_string(c.c) + "s" + std::to_string(c.s)
+    rep << (c.per_sm == 0 ? std::string(b->elem == 8 ? "default" : "resident") : c.G <= 1 ? "R" + std::to_string(c.w) + "x" + std::to_string(c.c) + "s" + std::to_string(c.s)
                      : "G" + std::to_string(c.G) + "/b" + std::to_string(c.blk))
         << "/x" << c.per_sm << ":" << static_cast<long long>(b->total_cells * 16 / t / 1e6) << " ";
     if (t < best) {

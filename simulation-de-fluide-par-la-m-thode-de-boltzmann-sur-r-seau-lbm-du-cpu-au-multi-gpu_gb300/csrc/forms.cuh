@@ -20,6 +20,9 @@ struct Form<float> {
     return make_collide_consts<float>(float(tau), float(fx), float(fy));
   }
 };
+// FP64 with its multiplications on the integer units, for the kernels that the automatic choice
+// takes (step kernels chosen by number keep the hardware's).
+using F64IntPhys = ExactPhys<ExactF64Int>;
 template <>
 struct Form<double> {
   using A = ExactF64;
@@ -47,6 +50,16 @@ struct Form<__nv_bfloat16> {
     return make_fast_consts(float(tau), float(fx), float(fy), kStoreScale16);
   }
 };
+
+// Blocks per SM of the FP64 ring's grid. The collision is bound by the FP64 pipe, so what costs is
+// an uneven last wave: more blocks than reside (two or three) let the scheduler hand out the
+// last tiles one by one (1024 x 512 with the hardware's multiplications: 2702 MLUPS with the
+// resident grid, 3065 with 6 per SM; with integer ones 4499 and, with 12 per SM, 4721).
+constexpr int kF64GridPerSm = 12;
+
+// Dynamic shared memory that keeps a kernel to `blocks` resident blocks per SM (228 KB per SM,
+// 1 KB of it reserved per block).
+inline size_t smem_for_blocks(int blocks) { return (228 * 1024 / static_cast<size_t>(blocks > 0 ? blocks : 1) - 1024) / 128 * 128; }
 
 inline constexpr int kCx[kQ] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
 inline constexpr int kCy[kQ] = {0, 0, 1, 0, -1, 1, 1, -1, -1};

@@ -22,6 +22,7 @@
 #include <cstdint>
 
 #include "collide.h"
+#include "mul64.h"
 
 namespace lbm_b200 {
 
@@ -113,6 +114,11 @@ struct ExactF64 {
     return a / b;
 #endif
   }
+};
+
+// ExactF64 with its multiplications on the integer units (mul64.h).
+struct ExactF64Int : ExactF64 {
+  static __host__ __device__ __forceinline__ double mul(double a, double b) { return mul64(a, b); }
 };
 
 // Exact FP32 arithmetic on two cells per instruction (packed add.rn.f32x2 / fma.rn.f32x2).

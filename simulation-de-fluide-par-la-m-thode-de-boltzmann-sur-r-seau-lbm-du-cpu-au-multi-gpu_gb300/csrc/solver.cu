@@ -71,9 +71,8 @@ Eq9<typename StoreTraits<ST>::T> step_inlet_eq(const lbm_solver* s) {
 template <class ST, bool kPacked>
 using PhysOf = std::conditional_t<kPacked, typename Form<ST>::PackedPhys, typename Form<ST>::Phys>;
 
-template <class ST, bool kOpen, int kVariant, bool kPacked = false>
+template <class ST, bool kOpen, int kVariant, class Phys = typename Form<ST>::Phys>
 int launch_steps_t(lbm_solver* s, int steps) {
-  using Phys = PhysOf<ST, kPacked>;
   using T = typename StoreTraits<ST>::T;
   constexpr int G = StoreTraits<ST>::kVec;
   StepArgs<ST, Phys> a{};
@@ -86,11 +85,16 @@ int launch_steps_t(lbm_solver* s, int steps) {
   for (int i = 0; i < kQ; ++i) a.eq_in[i] = e.v[i];
   a.sc = s->sc;
   const auto kernel = pull_step_kernel<ST, Phys, kOpen, kVariant>;
+  // FP64 with integer multiplications holds 141 registers: blocks of half the size let 12 warps
+  // reside instead of 8 and even out the last wave (300 x 300: 2.60k MLUPS with 256 threads).
+  constexpr bool kInt = std::is_same_v<Phys, F64IntPhys>;
+  const int block = kInt ? std::min(s->block, 128) : s->block;
   int grid = s->grid;
   if (grid <= 0) {
     int per_sm = 0;
-    LBM_CUDA(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, s->block, 0));
-    const int warps_per_block = s->block / 32;
+    LBM_CUDA(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0));
+    if (kInt) per_sm = kF64GridPerSm;
+    const int warps_per_block = block / 32;
     const int need = (a.items + warps_per_block - 1) / warps_per_block;
     grid = std::max(1, std::min(need, std::max(1, per_sm) * s->sm_count));
   }
@@ -100,7 +104,7 @@ int launch_steps_t(lbm_solver* s, int steps) {
     a.dst = static_cast<ST*>(s->buf[s->cur ^ 1]);
     a.step_ctr = s->step_ctr;
     a.step_off = static_cast<uint32_t>(k);
-    LBM_CUDA(s, launch_dependent(kernel, dim3(grid), dim3(s->block), 0, s->stream, a));
+    LBM_CUDA(s, launch_dependent(kernel, dim3(grid), dim3(block), 0, s->stream, a));
     s->cur ^= 1;
   }
   LBM_CUDA(s, cudaGetLastError());
@@ -188,20 +192,15 @@ int launch_async_t(lbm_solver* s, int steps) {
   return LBM_OK;
 }
 
-// Blocks per SM of the FP64 ring's grid. The collision is bound by the FP64 pipe, so what costs is
-// an uneven last wave: more blocks than reside (two or three) let the scheduler hand out the
-// last tiles one by one (1024 x 512: 2702 MLUPS with the resident grid, 3065 with 6 per SM).
-constexpr int kF64GridPerSm = 6;
-
 // Warp-specialised ring with one cell (plain FP32 / FP64) or one pair of cells (16-bit storage)
 // per lane (step_ring.cuh). kMaxBlocks > 0 caps the resident blocks per SM (by the shared memory
 // a block asks for): past the bytes in flight that cover the latency, more of them only queue in
 // front of HBM and cost bandwidth (FP32, 4096^2, variant 12: 87.1k MLUPS at the 3 blocks per SM
 // it was tuned for, 78.5k at the 4 its 56 registers allow).
-template <class ST, bool kOpen, int kW, int kC, int kStages, int kMinBlocks, int kMaxBlocks = 0>
+template <class ST, bool kOpen, int kW, int kC, int kStages, int kMinBlocks, int kMaxBlocks = 0,
+          class Phys = typename Form<ST>::Phys>
 int launch_ring_t(lbm_solver* s, int steps) {
   {
-    using Phys = typename Form<ST>::Phys;
     using T = typename StoreTraits<ST>::T;
     using S = RingShape<ST, kW, kC>;
     StepArgs<ST, Phys> a{};
@@ -215,8 +214,7 @@ int launch_ring_t(lbm_solver* s, int steps) {
     const int tiles = tpr * s->ny;
     const auto kernel = ring_step_kernel<ST, Phys, kOpen, kW, kC, kStages, kMinBlocks>;
     size_t smem = ring_smem_bytes<S>(kStages);
-    if (kMaxBlocks > 0)  // 228 KB per SM, 1 KB of it reserved per block
-      smem = std::max<size_t>(smem, (228 * 1024 / std::max(kMaxBlocks, 1) - 1024) / 128 * 128);
+    if (kMaxBlocks > 0) smem = std::max(smem, smem_for_blocks(kMaxBlocks));
     LBM_CUDA(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
     int grid = s->grid;
@@ -251,6 +249,10 @@ int launch_ring_t(lbm_solver* s, int steps) {
 // blocks 89.0k / 90.9k / 79k (3000 x 5000: 87.9k / 91.1k / 79k; 2048^2: 85.4k / 87.8k / 84.6k).
 constexpr int kVariantF32Large = 23;
 
+// Internal variants of the automatic choice in FP64: ring and direct kernel with integer
+// multiplications.
+constexpr int kVariantF64Ring = 25, kVariantF64Direct = 26;
+
 // Internal variant number of resident launches (step_resident.cuh). A launch loads and stores the
 // state and has no dependent-launch overlap, so short runs stay with the step kernels (us a step,
 // resident against them, runs of 2 / 3 / 4 / 16 / 400 steps: FP32 128 x 66 6.5 / 5.3 / 3.6 / 1.9 /
@@ -271,23 +273,20 @@ constexpr int kVariantResident = 24;
 // v22 170.3k), 8192^2 v17 175.7k (v20 168.9k), so grids of at least 2^25 cells take v17.
 // Rows narrower than 256 cells take the
 // direct kernel (0), whose 128-cell chunks leave fewer lanes idle than the rings' wide tiles
-// (FP64 on 100 x 2000: the ring 12 reached 1.0k MLUPS with a fifth of its lanes busy). FP64 is
-// bound by the FP64 pipe: whole 256-cell tiles take the ring whose tile count (512 or 256 cells)
-// spreads more evenly over the SMs (1024 x 256: 12 2661 MLUPS, 19 3012; 2048^2: 3217 both), rows
-// whose 256-cell tiles are less than 95 % full the direct kernel (700 x 333: 19 2701, 0 3047).
+// (FP64 on 100 x 2000: the ring 12 reached 1.0k MLUPS with a fifth of its lanes busy). FP64
+// takes kernels of its own, with the multiplications on the integer units (mul64.h), bound by the
+// FP64 pipe's additions: the ring with 256-cell tiles, 4 stages, 3 blocks per SM (MLUPS at
+// 1024 x 512: 2.56k with the hardware's multiplications and the resident grid, 3.07k with the
+// shorter collision and the larger grid, 4.72k with integer multiplications; 2048^2 4.90k; with
+// no force 6.02k), the direct kernel where the row's 256-cell tiles are less than 95 % full.
 template <class ST>
 int auto_variant(const lbm_solver* s) {
   using S = RingShape<ST, 8, 2>;
   const long long cells = static_cast<long long>(s->nx) * s->ny;
-  if (s->nx < 256) return 0;
+  if (s->nx < 256) return sizeof(ST) == 8 ? kVariantF64Direct : 0;
   if (sizeof(ST) == 8) {
-    const int half = S::TW / 2;
-    if (20LL * s->nx < 19LL * ((s->nx + half - 1) / half * half)) return 0;
-    auto spread = [&](int tw) {  // busy share of the SMs over all waves of tiles
-      const double tiles = static_cast<double>((s->nx + tw - 1) / tw) * s->ny;
-      return tiles / (std::ceil(tiles / s->sm_count) * s->sm_count);
-    };
-    return spread(half) > 1.01 * spread(S::TW) ? 19 : 12;
+    const int tw = S::TW / 2;
+    return 20LL * s->nx < 19LL * ((s->nx + tw - 1) / tw * tw) ? kVariantF64Direct : kVariantF64Ring;
   }
   if (sizeof(ST) == 2) {
     if (cells < (2LL << 20)) return 19;
@@ -300,6 +299,10 @@ int auto_variant(const lbm_solver* s) {
 template <class ST, bool kOpen>
 int launch_steps_o(lbm_solver* s, int steps) {
   s->last_variant = s->variant >= 0 ? s->variant : auto_variant<ST>(s);
+  if constexpr (sizeof(ST) == 8) {
+    if (s->last_variant == kVariantF64Ring) return launch_ring_t<ST, kOpen, 8, 1, 4, 3, 0, F64IntPhys>(s, steps);
+    if (s->last_variant == kVariantF64Direct) return launch_steps_t<ST, kOpen, 0, F64IntPhys>(s, steps);
+  }
   switch (s->last_variant) {
     case 1: return launch_steps_t<ST, kOpen, 1>(s, steps);
     case 2: return launch_steps_t<ST, kOpen, 2>(s, steps);
@@ -308,7 +311,7 @@ int launch_steps_o(lbm_solver* s, int steps) {
     case 5: return launch_tma_t<ST, kOpen, 3>(s, steps);
     case 6: return launch_tma_t<ST, kOpen, 4>(s, steps);
     case 7: return launch_tma_t<ST, kOpen, 2, true>(s, steps);
-    case 8: return launch_steps_t<ST, kOpen, 0, true>(s, steps);
+    case 8: return launch_steps_t<ST, kOpen, 0, PhysOf<ST, true>>(s, steps);
     case 9: return launch_async_t<ST, kOpen, 2>(s, steps);
     case 10: return launch_async_t<ST, kOpen, 3>(s, steps);
     case 11: return launch_async_t<ST, kOpen, 4>(s, steps);

@@ -19,6 +19,8 @@
 //   * warps whose cells are all solid skip the chunk (solid slots are never read).
 #pragma once
 
+#include <type_traits>
+
 #include "lbm_device.cuh"
 
 namespace lbm_b200 {
@@ -53,6 +55,41 @@ __device__ __forceinline__ uint32_t step_rkey(const StepArgs<ST, Phys>& p) {
   return sr_step_key(__ldg(p.step_ctr) + p.step_off);
 }
 
+// Is any of the values NaN (or infinite)?
+__device__ __forceinline__ bool any_nan(const double (&v)[kQ]) {
+  uint32_t top = 0;
+#pragma unroll
+  for (int i = 0; i < kQ; ++i) top = max(top, static_cast<uint32_t>(__double2hiint(v[i])) & 0x7fffffffu);
+  return top >= 0x7ff00000u;
+}
+
+// The collision with the hardware's multiplications, out of line, for the cells whose integer
+// ones gave NaN.
+template <class A>
+__device__ __noinline__ void collide_exact_rare(const typename A::T (&g)[kQ], CollideConsts<typename A::T> k,
+                                                typename A::T (&out)[kQ]) {
+  collide_exact_kind<A, kForceXY>(g, k, out);
+}
+
+// The collision of one cell as the step kernels take it. Integer multiplications (ExactF64Int)
+// give NaN for factors outside their range; such a cell, or one that holds a NaN, is collided
+// again with the hardware's.
+template <class A, int kForce>
+__device__ __forceinline__ void collide_cell(const typename A::T (&g)[kQ], const CollideConsts<typename A::T>& k,
+                                             typename A::T (&out)[kQ]) {
+  collide_exact_kind<A, kForce>(g, k, out);
+  if constexpr (std::is_same_v<A, ExactF64Int>) {
+    if (any_nan(out)) {
+      double v[kQ], o[kQ];
+#pragma unroll
+      for (int i = 0; i < kQ; ++i) v[i] = g[i];
+      collide_exact_rare<ExactF64>(v, k, o);
+#pragma unroll
+      for (int i = 0; i < kQ; ++i) out[i] = o[i];
+    }
+  }
+}
+
 // Exact (bit-for-bit with v0) physics, one cell at a time (FP64).
 template <class A>
 struct ExactPhys {
@@ -77,7 +114,7 @@ struct ExactPhys {
       T g[kQ], o[kQ];
 #pragma unroll
       for (int i = 0; i < kQ; ++i) g[i] = v[i][c];
-      collide_exact_kind<A, kForce>(g, k, o);
+      collide_cell<A, kForce>(g, k, o);
 #pragma unroll
       for (int i = 0; i < kQ; ++i) out[i][c] = o[i];
     }

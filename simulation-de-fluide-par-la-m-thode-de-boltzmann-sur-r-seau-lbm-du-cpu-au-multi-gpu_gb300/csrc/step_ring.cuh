@@ -138,7 +138,7 @@ __device__ __forceinline__ void ring_cell(const StepArgs<ST, ExactPhys<A>>& p, c
   (void)ym;
   (void)yp;
   T out[kQ];
-  collide_exact_kind<A, kForce>(v, p.k, out);
+  collide_cell<A, kForce>(v, p.k, out);
   ST* d = p.dst + static_cast<long long>(y) * p.g.pitch + x;
 #pragma unroll
   for (int i = 0; i < kQ; ++i) d[i * plane] = out[i];

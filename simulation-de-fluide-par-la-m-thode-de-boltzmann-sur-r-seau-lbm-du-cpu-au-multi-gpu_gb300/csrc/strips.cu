@@ -90,9 +90,9 @@ struct StripSplit {
 // strip, local row and first cell to the consumer warps in 16 bytes after the ring stage
 // (written before it arms the stage, read after the wait), so that eight consumer warps do not
 // repeat the divisions.
-template <class ST, class Phys, bool kOpen, int kC>
+template <class ST, class Phys, bool kOpen, int kW, int kC>
 struct StripPolicy {
-  using S = RingShape<ST, 8, kC>;
+  using S = RingShape<ST, kW, kC>;
   static constexpr bool kFinish = false;
   static constexpr int kStageBytes = S::kStageBytes + 16;
   const StepArgs<ST, Phys>& base;  // src / dst / mask: buffer bases; g: nx, pitch, mask words
@@ -134,30 +134,30 @@ struct StripPolicy {
 
 // Shared memory of a strip ring block: 2 stages of the policy, their barriers, then the strip
 // table when it is staged.
-template <class ST, class Phys, int kC>
+template <class ST, class Phys, int kW, int kC>
 __host__ __device__ constexpr size_t strip_ring_smem() {
-  return 2 * static_cast<size_t>(StripPolicy<ST, Phys, false, kC>::kStageBytes) + 4 * sizeof(uint64_t);
+  return 2 * static_cast<size_t>(StripPolicy<ST, Phys, false, kW, kC>::kStageBytes) + 4 * sizeof(uint64_t);
 }
 
-// One step of every strip: the solver's ring kernel (8 consumer warps x kC passes, 2 stages)
+// One step of every strip: the solver's ring kernel (kW consumer warps x kC passes, 2 stages)
 // over the strips' tiles, with the halo exchange fused into the stores of each strip's top and
 // bottom owned rows (the ghost rows of the destination buffer are complete when it ends).
-template <class ST, class Phys, bool kOpen, int kC, int kMinBlocks>
-__global__ void __launch_bounds__(32 * 9, kMinBlocks)
+template <class ST, class Phys, bool kOpen, int kW, int kC, int kMinBlocks>
+__global__ void __launch_bounds__(32 * (kW + 1), kMinBlocks)
     strip_ring_kernel(const StepArgs<ST, Phys> base, const StripTile* __restrict__ tab, int strips,
                       const StripSplit split, FastDiv tpr, int tiles, int reverse, int* err) {
-  using Pol = StripPolicy<ST, Phys, kOpen, kC>;
+  using Pol = StripPolicy<ST, Phys, kOpen, kW, kC>;
   extern __shared__ __align__(128) unsigned char smem[];
   grid_dependency_wait();
   const StripTile* t = tab;
   if (strips <= kStripTableSmem) {
-    StripTile* s_tab = reinterpret_cast<StripTile*>(smem + strip_ring_smem<ST, Phys, kC>());
+    StripTile* s_tab = reinterpret_cast<StripTile*>(smem + strip_ring_smem<ST, Phys, kW, kC>());
     for (int k = threadIdx.x; k < strips; k += blockDim.x) s_tab[k] = tab[k];
     __syncthreads();
     t = s_tab;
   }
   const Pol pol{base, t, split, tpr, tiles, reverse};
-  tile_pipeline<8, 2, Pol::kStageBytes>(smem, pol, tiles, err);
+  tile_pipeline<kW, 2, Pol::kStageBytes>(smem, pol, tiles, err);
 }
 
 // Device halo exchange of all strips (raw elements E, the storage bits): thread per
@@ -274,24 +274,27 @@ int halo_t(lbm_strips* h, int b) {
 }
 
 // `steps` steps: one ring launch per step over every strip's owned rows (halo fused); then the
-// step counter advances. kC: ring passes per strip (the solver's variant 12 / 17 shape, or
-// variant 20's for 16-bit storage on wide rows).
-template <class ST, bool kOpen, int kC>
+// step counter advances. Ring shape kW consumer warps x kC passes: FP32 8 x 2, and the solver's
+// for large grids there (4 x 2, 5 resident blocks), FP64 8 x 1 with integer multiplications and 3 blocks, 16-bit
+// storage 8 x 2, or 8 x 4 on wide rows.
+template <class ST, bool kOpen, int kW, int kC>
 int steps_tc(lbm_strips* h, int steps) {
-  using Phys = typename Form<ST>::Phys;
+  using Phys = std::conditional_t<sizeof(ST) == 8, F64IntPhys, typename Form<ST>::Phys>;
   using T = typename StoreTraits<ST>::T;
-  // Register caps: 3 resident blocks (72 registers); 2 for the four-pass shape with open x
-  // boundaries (it would spill at 72); none in FP64.
-  constexpr int kMin = sizeof(ST) == 8 ? 1 : ((kC == 4 && kOpen) ? 2 : 3);
-  using S = RingShape<ST, 8, kC>;
-  const auto kernel = strip_ring_kernel<ST, Phys, kOpen, kC, kMin>;
-  const size_t smem = strip_ring_smem<ST, Phys, kC>() +
-                      (h->strips <= kStripTableSmem ? h->strips * sizeof(StripTile) : 0);
+  // Register caps: 3 resident blocks of 9 warps (72 registers), 5 of 5 warps; 2 for the four-pass
+  // shape with open x boundaries (it would spill at 72).
+  constexpr int kMin = kW == 4 ? 5 : ((kC == 4 && kOpen) ? 2 : 3);
+  using S = RingShape<ST, kW, kC>;
+  const auto kernel = strip_ring_kernel<ST, Phys, kOpen, kW, kC, kMin>;
+  size_t smem = strip_ring_smem<ST, Phys, kW, kC>() +
+                (h->strips <= kStripTableSmem ? h->strips * sizeof(StripTile) : 0);
+  if (kW == 4) smem = std::max(smem, smem_for_blocks(kMin));  // no more than kMin blocks
   S_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   int per_sm = 0;
   S_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, S::kThreads, smem));
   const int tpr = (h->nx + S::TW - 1) / S::TW;
   const int tiles = tpr * h->ny;  // the strips' owned rows cover the lattice once
+  if (sizeof(ST) == 8) per_sm = kF64GridPerSm;
   const int grid = std::max(1, std::min(tiles, std::max(1, per_sm) * h->sm_count));
   const Eq9<T> e = strip_inlet<ST>(h, true);
   StepArgs<ST, Phys> a{};
@@ -324,9 +327,16 @@ int steps_tc(lbm_strips* h, int steps) {
 template <class ST, bool kOpen>
 int steps_t(lbm_strips* h, int steps) {
   if constexpr (sizeof(ST) == 2) {
-    if (h->passes == 4) return steps_tc<ST, kOpen, 4>(h, steps);
+    if (h->passes == 4) return steps_tc<ST, kOpen, 8, 4>(h, steps);
+    return steps_tc<ST, kOpen, 8, 2>(h, steps);
+  } else if constexpr (sizeof(ST) == 8) {
+    return steps_tc<ST, kOpen, 8, 1>(h, steps);
+  } else {
+    // (2048^2, 5 strips: 85.5k MLUPS with the narrow tiles, 84.5k with the wide ones; 400^2: 28.8k
+    // and 31.4k.)
+    if (static_cast<long long>(h->nx) * h->ny >= (2LL << 20)) return steps_tc<ST, kOpen, 4, 2>(h, steps);
+    return steps_tc<ST, kOpen, 8, 2>(h, steps);
   }
-  return steps_tc<ST, kOpen, 2>(h, steps);
 }
 
 template <class ST>
