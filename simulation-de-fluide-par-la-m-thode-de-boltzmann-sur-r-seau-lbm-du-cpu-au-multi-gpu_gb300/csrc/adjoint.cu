@@ -277,11 +277,35 @@ __device__ __forceinline__ void issue_pull(unsigned char* st, unsigned char* wra
   }
 }
 
+// Adds v to *slot, which no other thread of the launch touches, without waiting for its old value.
+__device__ __forceinline__ void add_to(double* slot, double v) {
+  asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(slot), "d"(v) : "memory");
+}
 // Warp sum (fixed shuffle tree) of one value per lane, added by lane 0 to *slot.
 __device__ __forceinline__ void warp_add_to(double v, double* slot, int lane) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (lane == 0) *slot += v;
+  if (lane == 0) add_to(slot, v);
+}
+// The same for three values into slot[0 .. 2]. The values are spread over the lanes as the tree
+// narrows (lanes with bit 4 clear go on with a and half of c, the others with b and half of c, then
+// bit 3 splits c off), so that a warp spends 6 double additions instead of 15: at two per SM and
+// cycle, the 24 consumer warps' sums at the end of a launch were 3.6 us of the FP64 pipe.
+__device__ __forceinline__ void warp_add3_to(double a, double b, double c, double* slot, int lane) {
+  const bool hi = lane & 16;
+  // a (low half) or b (high half), each the sum over the lane pair; c over the pair in both.
+  double ab = (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, 16);
+  c += __shfl_xor_sync(0xffffffffu, c, 16);
+  // Within each half of 16: lanes with bit 3 clear take ab, the others of the low half take c.
+  const bool lo8 = !(lane & 8);
+  const double ab2 = __shfl_xor_sync(0xffffffffu, ab, 8), c2 = __shfl_xor_sync(0xffffffffu, c, 8);
+  double v = lo8 ? ab + ab2 : c + c2;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  // lane 0: a, lane 16: b, lane 8: c.
+  if (lane == 0) add_to(slot, v);
+  if (lane == 16) add_to(slot + 1, v);
+  if (lane == 8) add_to(slot + 2, v);
 }
 
 // Slot of (instance b, this block, consumer warp cw).
@@ -405,6 +429,7 @@ template <class A, int kC, int kStages, int kMinBlocks>
 __global__ void __launch_bounds__(kAdjThreads, kMinBlocks)
     adj_forward_kernel(const FwdArgs<typename A::T> p, int* err) {
   extern __shared__ __align__(128) unsigned char smem[];
+  pipeline_init<kAdjW, kStages, FwdStage<typename A::T, kC>::kBytes>(smem);
   grid_dependency_wait();
   AdjForward<A, kC> pol{p};
   tile_pipeline<kAdjW, kStages, FwdStage<typename A::T, kC>::kBytes, kAdjProd>(smem, pol, p.at.total, err);
@@ -557,10 +582,8 @@ struct AdjBackward {
 
   __device__ __forceinline__ void flush(int cw, int lane) {
     if (cur_b >= 0) {
-      double* slot = p.grads + 3 * warp_slot(cur_b, cw);
-      warp_add_to(static_cast<double>(go), slot + 0, lane);
-      warp_add_to(static_cast<double>(gx), slot + 1, lane);
-      warp_add_to(static_cast<double>(gy), slot + 2, lane);
+      warp_add3_to(static_cast<double>(go), static_cast<double>(gx), static_cast<double>(gy),
+                   p.grads + 3 * warp_slot(cur_b, cw), lane);
     }
     go = gx = gy = T(0);
   }
@@ -652,6 +675,7 @@ template <class T, int kC, int kStages, int kMinBlocks>
 __global__ void __launch_bounds__(kAdjThreads, kMinBlocks)
     adj_backward_kernel(const BwdArgs<T> p, int* err) {
   extern __shared__ __align__(128) unsigned char smem[];
+  pipeline_init<kAdjW, kStages, BwdStage<T, kC>::kBytes>(smem);
   grid_dependency_wait();
   AdjBackward<T, kC> pol{p};
   tile_pipeline<kAdjW, kStages, BwdStage<T, kC>::kBytes, kAdjProd>(smem, pol, p.at.total, err);
@@ -771,7 +795,8 @@ struct lbm_adjoint {
   void* state[2] = {nullptr, nullptr};
   void* ckpt = nullptr;          // checkpoints: (T/K + 1) states
   size_t ckpt_count = 0;
-  void* seg = nullptr;           // K recomputed states (a segment's first state is its checkpoint)
+  void* seg = nullptr;           // K states of a segment (its first state is its checkpoint)
+  bool seg_last = false;         // seg holds the last forward run's last segment
   void* ybar[2] = {nullptr, nullptr};
   double* abar = nullptr;        // batch pitched planes
   void* aseg = nullptr;          // batch pitched planes, per-segment alpha_bar in the state precision
@@ -838,12 +863,12 @@ struct AdjKernels {
   static constexpr auto bwd = adj_backward_kernel<T, kC, LC::kBwdStages, LC::kBwdMin>;
 };
 
-// Automatic cells per lane. Forward (FP32): the tile width (256 or 512 cells) that leaves fewer
-// idle lanes in a row, the wider one on a tie (half the per-tile work per cell). Backward and
-// FP64: one cell per lane (a 512-cell backward stage needs 42 KB, which leaves two blocks of 16
-// consumer warps per SM instead of three of 24).
-int auto_cells(const lbm_adjoint* a, bool backward) {
-  if (a->precision == LBM_FP64 || backward) return 1;
+// Automatic cells per lane. FP32: the tile width (256 or 512 cells) that leaves fewer idle lanes
+// in a row, the wider one on a tie (half the per-tile work per cell). 512 x 128, 8 / 16 / 32
+// instances, us per backward step with 256-cell and 512-cell backward tiles: 25.6 / 39.1 / 69.1
+// and 23.4 / 37.8 / 68.2. FP64: one cell per lane.
+int auto_cells(const lbm_adjoint* a) {
+  if (a->precision == LBM_FP64) return 1;
   const int nx = a->g.nx;
   const int w1 = (nx + 255) / 256 * 256 - nx, w2 = (nx + 511) / 512 * 512 - nx;
   return w2 <= w1 ? 2 : 1;
@@ -880,8 +905,8 @@ int sweep_grid(lbm_adjoint* a, K kernel, size_t smem, int cells, int* grid) {
 template <class A>
 int configure(lbm_adjoint* a) {
   using T = typename A::T;
-  const int fc = a->fwd_req ? a->fwd_req : auto_cells(a, false);
-  const int bc = a->bwd_req ? a->bwd_req : auto_cells(a, true);
+  const int fc = a->fwd_req ? a->fwd_req : auto_cells(a);
+  const int bc = a->bwd_req ? a->bwd_req : auto_cells(a);
   int rc = with_shape<T>(fc, [&](auto kc) {
     using LC = AdjLaunch<T, decltype(kc)::value>;
     return sweep_grid(a, AdjKernels<A, decltype(kc)::value>::fwd, LC::fwd_smem(), decltype(kc)::value, &a->fwd_grid);
@@ -1058,6 +1083,9 @@ int forward_t(lbm_adjoint* a, const void* s0_host, int steps, int window, double
   const int nhalf = adj_halves(a);
   FwdHalf<T> half[2];
   for (int k = 0; k < nhalf; ++k) half[k] = fwd_half<A>(a, p, k);
+  a->seg_last = false;
+  char* seg = static_cast<char*>(a->seg);
+  const int t_last = (steps - 1) / a->K * a->K;  // first state of the last segment
   const void* cur = ckpt;
   int spare = 0;
   ADJ_CUDA(a, cudaEventRecord(a->ev[0], a->stream));
@@ -1065,10 +1093,13 @@ int forward_t(lbm_adjoint* a, const void* s0_host, int steps, int window, double
   for (int t = 0; t < steps; ++t) {
     const bool in_window = t >= steps - window + 1;
     const bool is_ckpt = (t + 1) % a->K == 0;
-    void* out = is_ckpt ? ckpt + static_cast<size_t>((t + 1) / a->K) * sb : a->state[spare];
+    // (The final state stays out of the segment buffer, which the backward run overwrites.)
+    const bool to_seg = !is_ckpt && seg && t >= t_last && t + 1 < steps;
+    void* out = is_ckpt ? ckpt + static_cast<size_t>((t + 1) / a->K) * sb
+                        : (to_seg ? seg + static_cast<size_t>(t - t_last) * sb : a->state[spare]);
     for (int k = 0; k < nhalf; ++k)
       if (const int rc = launch_forward<A>(a, half[k], cur, out, in_window ? a->obj_part : nullptr, t & 1)) return rc;
-    if (!is_ckpt) spare ^= 1;
+    if (!is_ckpt && !to_seg) spare ^= 1;
     cur = out;
   }
   if (nhalf == 2) ADJ_CUDA(a, adj_join(a, a->stream2, a->stream));
@@ -1088,6 +1119,7 @@ int forward_t(lbm_adjoint* a, const void* s0_host, int steps, int window, double
   a->steps = steps;
   a->window = window;
   a->have_forward = true;
+  a->seg_last = seg != nullptr;
   a->fin = cur;
   return LBM_OK;
 }
@@ -1156,10 +1188,16 @@ int backward_t(lbm_adjoint* a, double* dtau, double* dfx, double* dfy, double* d
   const int nseg = (T_steps + K - 1) / K;
   for (int s = nseg - 1; s >= 0; --s) {
     const int t0 = s * K, t1 = std::min(T_steps, t0 + K);
-    // R_{t0} is checkpoint s; recompute R_{t0 + 1 .. t1} into seg[0 .. t1 - t0 - 1].
+    // R_{t0} is checkpoint s, R_T the forward run's final state; recompute R_{t0 + 1 .. t1} into
+    // seg[0 .. t1 - t0 - 1] unless the forward run left them there.
     const char* base = static_cast<const char*>(a->ckpt) + static_cast<size_t>(s) * sb;
-    auto state_at = [&](int t) -> const void* { return t == t0 ? base : seg + static_cast<size_t>(t - t0 - 1) * sb; };
-    for (int t = t0; t < t1; ++t)
+    const bool kept = a->seg_last && s == nseg - 1;
+    auto state_at = [&](int t) -> const void* {
+      if (t == t0) return base;
+      return kept && t == T_steps ? a->fin : seg + static_cast<size_t>(t - t0 - 1) * sb;
+    };
+    if (!kept) a->seg_last = false;
+    for (int t = t0; t < t1 && !kept; ++t)
       for (int k = 0; k < nhalf; ++k)
         if (const int rc = launch_forward<A>(a, fh[k], state_at(t), seg + static_cast<size_t>(t - t0) * sb, nullptr, t & 1))
           return rc;

@@ -395,6 +395,7 @@ __global__ void __launch_bounds__(FlatShape<ST, kW, kC>::kThreads, (batch_ring_m
     batch_ring_kernel(const BatchArgs<ST, Phys> a, int tiles, int* err) {
   using Pol = BatchFlatPolicy<ST, Phys, kW, kC>;
   extern __shared__ __align__(128) unsigned char smem[];
+  pipeline_init<kW, kStages, Pol::kStageBytes>(smem);
   grid_dependency_wait();
   Pol pol{a, sizeof(ST) == 2 ? sr_step_key(__ldg(a.step) + a.step_off) : 0u};
   tile_pipeline<kW, kStages, Pol::kStageBytes, FlatShape<ST, kW, kC>::kProd>(smem, pol, tiles, err);

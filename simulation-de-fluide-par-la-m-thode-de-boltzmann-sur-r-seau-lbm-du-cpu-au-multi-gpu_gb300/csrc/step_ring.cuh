@@ -409,13 +409,13 @@ struct warp_issue<P, std::void_t<decltype(P::kWarpIssue)>> : std::bool_constant<
 // pol.finish(cw, lane), also after a wait ran out (the host then reports the timeout), e.g. to
 // write the warp's partial sums. Warps never synchronise with one another after the start, so
 // a wait that ran out in one warp cannot leave another waiting at a barrier.
-template <int kW, int kStages, int kStageBytes, int kProd = 1, class Pol>
-__device__ __forceinline__ void tile_pipeline(unsigned char* smem, Pol& pol, int tiles, int* err) {
-  static_assert(kProd >= 1 && kStages >= 1, "at least one producer warp and one stage");
-  static_assert(kProd <= kStages, "a stage's barrier may run two phases behind a producer otherwise");
+//
+// pipeline_init sets up the ring's barriers; kernels call it before grid_dependency_wait, so that
+// it overlaps the previous step's drain.
+template <int kW, int kStages, int kStageBytes>
+__device__ __forceinline__ void pipeline_init(unsigned char* smem) {
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + static_cast<size_t>(kStages) * kStageBytes);
   uint64_t* empty = full + kStages;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
@@ -424,6 +424,15 @@ __device__ __forceinline__ void tile_pipeline(unsigned char* smem, Pol& pol, int
     mbar_fence_init();
   }
   __syncthreads();
+}
+
+template <int kW, int kStages, int kStageBytes, int kProd = 1, class Pol>
+__device__ __forceinline__ void tile_pipeline(unsigned char* smem, Pol& pol, int tiles, int* err) {
+  static_assert(kProd >= 1 && kStages >= 1, "at least one producer warp and one stage");
+  static_assert(kProd <= kStages, "a stage's barrier may run two phases behind a producer otherwise");
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + static_cast<size_t>(kStages) * kStageBytes);
+  uint64_t* empty = full + kStages;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (warp < kProd) {
     constexpr bool kWarp = warp_issue<Pol>::value;
@@ -567,6 +576,7 @@ __global__ void __launch_bounds__(32 * (kW + 1), kMinBlocks)
     ring_step_kernel(const StepArgs<ST, Phys> p, int tiles_per_row, int tiles, int row0, int reverse, int* err) {
   using S = RingShape<ST, kW, kC>;
   extern __shared__ __align__(128) unsigned char smem[];
+  pipeline_init<kW, kStages, S::kStageBytes>(smem);
   grid_dependency_wait();
   const GridTiles<ST, Phys, S::TW> grid_tiles{p, tiles_per_row, row0, tiles, reverse};
   ring_pipeline<ST, Phys, kOpen, kW, kC, kStages>(smem, grid_tiles, tiles, err);

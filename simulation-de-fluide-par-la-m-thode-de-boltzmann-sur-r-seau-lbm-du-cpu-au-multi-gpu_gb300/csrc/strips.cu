@@ -148,14 +148,14 @@ __global__ void __launch_bounds__(32 * (kW + 1), kMinBlocks)
                       const StripSplit split, FastDiv tpr, int tiles, int reverse, int* err) {
   using Pol = StripPolicy<ST, Phys, kOpen, kW, kC>;
   extern __shared__ __align__(128) unsigned char smem[];
-  grid_dependency_wait();
   const StripTile* t = tab;
-  if (strips <= kStripTableSmem) {
+  if (strips <= kStripTableSmem) {  // (no step writes the table)
     StripTile* s_tab = reinterpret_cast<StripTile*>(smem + strip_ring_smem<ST, Phys, kW, kC>());
     for (int k = threadIdx.x; k < strips; k += blockDim.x) s_tab[k] = tab[k];
-    __syncthreads();
     t = s_tab;
   }
+  pipeline_init<kW, 2, Pol::kStageBytes>(smem);
+  grid_dependency_wait();
   const Pol pol{base, t, split, tpr, tiles, reverse};
   tile_pipeline<kW, 2, Pol::kStageBytes>(smem, pol, tiles, err);
 }
