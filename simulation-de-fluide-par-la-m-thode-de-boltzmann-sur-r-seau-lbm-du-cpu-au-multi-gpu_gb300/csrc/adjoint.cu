@@ -43,6 +43,7 @@
 #include "lbm_device.cuh"
 #include "solver_internal.h"
 #include "fastdiv.h"
+#include "host_access.h"
 #include "step_ring.cuh"
 
 using namespace lbm_b200;
@@ -743,30 +744,40 @@ __global__ void adj_set_state_kernel(T* __restrict__ R, const uint32_t* __restri
   }
 }
 
-// v0-layout post-streaming state of instance b (pull gather of its pitched state).
+// v0-layout post-streaming state of instance b (pull gather of its pitched state), by contiguous
+// runs of a block's cells.
 template <class T>
-__global__ void adj_get_state_kernel(const T* __restrict__ R, const uint32_t* __restrict__ mask,
-                                     const AdjGeom g, int b, T* __restrict__ aos) {
+__global__ void __launch_bounds__(kAuxThreads)
+    adj_get_state_kernel(const T* __restrict__ R, const uint32_t* __restrict__ mask, const AdjGeom g, int b,
+                         T* __restrict__ aos) {
+  __shared__ T run[kAuxThreads * kQ];
   const long long n = static_cast<long long>(g.nx) * g.ny;
   const T* Rb = R + b * g.inst;
-  for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
-       c += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int y = static_cast<int>(c / g.nx), x = static_cast<int>(c - static_cast<long long>(y) * g.nx);
-    const long long own = static_cast<long long>(y) * g.pitch + x;
-    const bool solid = mask_solid(mask, g.mask_words, x, y);
+  for (long long c0 = static_cast<long long>(blockIdx.x) * kAuxThreads; c0 < n;
+       c0 += static_cast<long long>(gridDim.x) * kAuxThreads) {
+    const long long c = c0 + threadIdx.x;
+    const int cells = static_cast<int>(n - c0 < kAuxThreads ? n - c0 : kAuxThreads);
+    if (c < n) {
+      const int y = static_cast<int>(c / g.nx), x = static_cast<int>(c - static_cast<long long>(y) * g.nx);
+      const long long own = static_cast<long long>(y) * g.pitch + x;
+      const bool solid = mask_solid(mask, g.mask_words, x, y);
 #pragma unroll
-    for (int i = 0; i < kQ; ++i) {
-      T s = T(0);
-      if (!solid) {
-        int xs = x - dir_cx(i), ys = y - dir_cy(i);
-        xs = xs < 0 ? g.nx - 1 : (xs >= g.nx ? 0 : xs);
-        ys = ys < 0 ? g.ny - 1 : (ys >= g.ny ? 0 : ys);
-        s = mask_solid(mask, g.mask_words, xs, ys)
-                ? Rb[dir_opp(i) * g.plane + own]
-                : Rb[i * g.plane + static_cast<long long>(ys) * g.pitch + xs];
+      for (int i = 0; i < kQ; ++i) {
+        T s = T(0);
+        if (!solid) {
+          int xs = x - dir_cx(i), ys = y - dir_cy(i);
+          xs = xs < 0 ? g.nx - 1 : (xs >= g.nx ? 0 : xs);
+          ys = ys < 0 ? g.ny - 1 : (ys >= g.ny ? 0 : ys);
+          s = mask_solid(mask, g.mask_words, xs, ys)
+                  ? Rb[dir_opp(i) * g.plane + own]
+                  : Rb[i * g.plane + static_cast<long long>(ys) * g.pitch + xs];
+        }
+        run[threadIdx.x * kQ + i] = s;
       }
-      aos[c * kQ + i] = s;
     }
+    __syncthreads();
+    for (int k = threadIdx.x; k < cells * kQ; k += kAuxThreads) aos[c0 * kQ + k] = run[k];
+    __syncthreads();
   }
 }
 
@@ -782,6 +793,16 @@ __global__ void to_pitched_kernel(const double* __restrict__ in, T* __restrict__
   }
 }
 
+// The reverse for FP64 fields: pitched -> unpadded.
+__global__ void from_pitched_kernel(const double* __restrict__ in, double* __restrict__ out, const AdjGeom g) {
+  const long long n = static_cast<long long>(g.nx) * g.ny;
+  for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < g.batch * n;
+       k += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long b = k / n, c = k - b * n;
+    const int y = static_cast<int>(c / g.nx), x = static_cast<int>(c - static_cast<long long>(y) * g.nx);
+    out[k] = in[b * g.plane + static_cast<long long>(y) * g.pitch + x];
+  }
+}
 
 }  // namespace
 
@@ -819,6 +840,7 @@ struct lbm_adjoint {
   cudaEvent_t join = nullptr;      // orders the two halves' streams
   double fwd_step_s = 0, bwd_step_s = 0;
   int sm_count = 0;
+  bool direct = false;  // kernels reach host memory
   std::string err;
 };
 
@@ -838,6 +860,16 @@ int adj_fail(lbm_adjoint* a, int code, const std::string& msg) {
                       std::string(#call) + ": " + cudaGetErrorString(e_));                   \
     }                                                                                        \
   } while (0)
+
+int ensure_stage(lbm_adjoint* a, size_t bytes) {
+  if (a->stage_bytes >= bytes) return LBM_OK;
+  cudaFree(a->stage);
+  a->stage = nullptr;
+  a->stage_bytes = 0;
+  ADJ_CUDA(a, cudaMalloc(&a->stage, bytes));
+  a->stage_bytes = bytes;
+  return LBM_OK;
+}
 
 size_t state_bytes(const lbm_adjoint* a) {
   return static_cast<size_t>(a->batch) * a->g.inst * a->elem;
@@ -1065,12 +1097,7 @@ int forward_t(lbm_adjoint* a, const void* s0_host, int steps, int window, double
   char* ckpt = static_cast<char*>(a->ckpt);
   if (s0_host) {
     const size_t hb = static_cast<size_t>(a->batch) * kQ * a->g.nx * a->g.ny * sizeof(T);
-    if (a->stage_bytes < hb) {
-      cudaFree(a->stage);
-      a->stage = nullptr;
-      ADJ_CUDA(a, cudaMalloc(&a->stage, hb));
-      a->stage_bytes = hb;
-    }
+    if (const int rc = ensure_stage(a, hb)) return rc;
     ADJ_CUDA(a, cudaMemcpyAsync(a->stage, s0_host, hb, cudaMemcpyHostToDevice, a->stream));
     adj_set_state_kernel<T><<<dim3(2 * a->sm_count, a->batch), kAuxThreads, 0, a->stream>>>(
         reinterpret_cast<T*>(ckpt), a->mask_d, a->g, static_cast<const T*>(a->stage));
@@ -1222,7 +1249,11 @@ int backward_t(lbm_adjoint* a, double* dtau, double* dfx, double* dfy, double* d
   if (nhalf == 2) ADJ_CUDA(a, adj_join(a, a->stream2, a->stream));
   ADJ_CUDA(a, cudaEventRecord(a->ev[1], a->stream));
   ADJ_CUDA(a, cudaGetLastError());
-  if (dalpha)
+  const size_t dalpha_bytes = static_cast<size_t>(a->batch) * a->g.nx * a->g.ny * sizeof(double);
+  if (double* view = dalpha ? static_cast<double*>(host_view(dalpha, dalpha_bytes, 8, a->direct, true)) : nullptr) {
+    from_pitched_kernel<<<4 * a->sm_count, kAuxThreads, 0, a->stream>>>(a->abar, view, a->g);
+    ADJ_CUDA(a, cudaGetLastError());
+  } else if (dalpha)
     ADJ_CUDA(a, cudaMemcpy2DAsync(dalpha, a->g.nx * sizeof(double), a->abar, a->g.pitch * sizeof(double),
                                   a->g.nx * sizeof(double), static_cast<size_t>(a->batch) * a->g.ny,
                                   cudaMemcpyDeviceToHost, a->stream));
@@ -1243,15 +1274,16 @@ int backward_t(lbm_adjoint* a, double* dtau, double* dfx, double* dfy, double* d
 template <class T>
 int get_state_t(lbm_adjoint* a, int b, void* host) {
   const size_t bytes = static_cast<size_t>(kQ) * a->g.nx * a->g.ny * sizeof(T);
-  if (a->stage_bytes < bytes) {
-    cudaFree(a->stage);
-    a->stage = nullptr;
-    ADJ_CUDA(a, cudaMalloc(&a->stage, bytes));
-    a->stage_bytes = bytes;
+  void* dst = host_view(host, bytes, sizeof(T), a->direct, true);
+  const bool in_place = dst != nullptr;
+  if (!in_place) {
+    if (const int rc = ensure_stage(a, bytes)) return rc;
+    dst = a->stage;
   }
   adj_get_state_kernel<T><<<2 * a->sm_count, kAuxThreads, 0, a->stream>>>(
-      static_cast<const T*>(a->fin), a->mask_d, a->g, b, static_cast<T*>(a->stage));
-  ADJ_CUDA(a, cudaMemcpyAsync(host, a->stage, bytes, cudaMemcpyDeviceToHost, a->stream));
+      static_cast<const T*>(a->fin), a->mask_d, a->g, b, static_cast<T*>(dst));
+  ADJ_CUDA(a, cudaGetLastError());
+  if (!in_place) ADJ_CUDA(a, cudaMemcpyAsync(host, a->stage, bytes, cudaMemcpyDeviceToHost, a->stream));
   ADJ_CUDA(a, cudaStreamSynchronize(a->stream));
   return LBM_OK;
 }
@@ -1303,6 +1335,7 @@ int lbm_adj_create(int nx, int ny, const uint8_t* solid, double tau, double fx, 
       cudaEventCreate(&a->ev[0]) != cudaSuccess || cudaEventCreate(&a->ev[1]) != cudaSuccess)
     return fail(LBM_ERR_CUDA);
   if (const int rc = precision == LBM_FP64 ? configure<ExactF64Int>(a) : configure<ExactF32>(a)) return fail(rc);
+  a->direct = host_memory_direct(dev);
   std::vector<uint32_t> words;
   pack_mask(solid, nx, ny, a->g.mask_words, words);
   const size_t sb = state_bytes(a);
@@ -1374,20 +1407,23 @@ int lbm_adj_set_alpha(lbm_adjoint* a, const double* alpha) {
     return LBM_OK;
   }
   const size_t n = static_cast<size_t>(a->batch) * a->g.nx * a->g.ny;
-  double* tmp = nullptr;
   if (!a->alpha) {
     ADJ_CUDA(a, cudaMalloc(&a->alpha, field_bytes_all(a, a->elem)));
     ADJ_CUDA(a, cudaMemsetAsync(a->alpha, 0, field_bytes_all(a, a->elem), a->stream));  // row padding
   }
-  ADJ_CUDA(a, cudaMalloc(&tmp, n * sizeof(double)));
-  ADJ_CUDA(a, cudaMemcpyAsync(tmp, alpha, n * sizeof(double), cudaMemcpyHostToDevice, a->stream));
+  // Read in place where kernels can address it, else through the staging buffer.
+  const double* src = static_cast<const double*>(host_view(alpha, n * sizeof(double), 8, a->direct, false));
+  if (!src) {
+    if (const int rc = ensure_stage(a, n * sizeof(double))) return rc;
+    ADJ_CUDA(a, cudaMemcpyAsync(a->stage, alpha, n * sizeof(double), cudaMemcpyHostToDevice, a->stream));
+    src = static_cast<const double*>(a->stage);
+  }
   if (a->precision == LBM_FP64)
-    to_pitched_kernel<double><<<2 * a->sm_count, kAuxThreads, 0, a->stream>>>(tmp, static_cast<double*>(a->alpha), a->g);
+    to_pitched_kernel<double><<<4 * a->sm_count, kAuxThreads, 0, a->stream>>>(src, static_cast<double*>(a->alpha), a->g);
   else
-    to_pitched_kernel<float><<<2 * a->sm_count, kAuxThreads, 0, a->stream>>>(tmp, static_cast<float*>(a->alpha), a->g);
-  const cudaError_t e = cudaStreamSynchronize(a->stream);
-  cudaFree(tmp);
-  if (e != cudaSuccess) return adj_fail(a, LBM_ERR_CUDA, cudaGetErrorString(e));
+    to_pitched_kernel<float><<<4 * a->sm_count, kAuxThreads, 0, a->stream>>>(src, static_cast<float*>(a->alpha), a->g);
+  ADJ_CUDA(a, cudaGetLastError());
+  ADJ_CUDA(a, cudaStreamSynchronize(a->stream));  // the host buffer may be reused on return
   a->have_forward = false;
   return LBM_OK;
 }

@@ -30,6 +30,7 @@
 #include "lbm_b200.h"
 #include "solver_internal.h"
 #include "forms.cuh"
+#include "host_access.h"
 #include "fastdiv.h"
 #include "step_kernel.cuh"
 #include "step_resident.cuh"
@@ -509,6 +510,7 @@ struct lbm_batch {
   size_t res_inst_at = 0, res_out_at = 0;
   bool chosen = false;
   int sm_count = 0, device = 0;
+  bool direct = false;  // kernels reach host memory
   std::string err, tune_report;
 };
 
@@ -920,7 +922,9 @@ int plan_resident(lbm_batch* b) {
       b->total_cells > static_cast<long long>(b->sm_count) * (kResPlaneBytes / kElem))
     return LBM_OK;
   std::vector<ResLayout> cut(b->count), best;
-  int lo = 1, hi = kResMaxItems;  // fewest items that fit, by bisection (fewer items, more tiles)
+  // The fewest items that fit, by bisection (fewer items, more tiles), from the even share on.
+  const long long per_item = kElem == 2 ? 64 : 32;
+  int lo = static_cast<int>(std::max<long long>(1, b->total_cells / per_item / b->sm_count)), hi = kResMaxItems;
   while (lo <= hi) {
     const int items = (lo + hi) / 2;
     long long tiles = 0;
@@ -951,10 +955,12 @@ int plan_resident(lbm_batch* b) {
   b->res_inst_at = up(blocks.size() * sizeof(ResBlock));
   b->res_out_at = b->res_inst_at + up(insts.size() * sizeof(ResInst));
   const size_t out_bytes = static_cast<size_t>(words) * sizeof(LLWord);
+  std::vector<char> tables(b->res_out_at);
+  std::memcpy(tables.data(), blocks.data(), blocks.size() * sizeof(ResBlock));
+  std::memcpy(tables.data() + b->res_inst_at, insts.data(), insts.size() * sizeof(ResInst));
   B_CUDA(b, cudaMalloc(&b->res_d, b->res_out_at + out_bytes));
-  B_CUDA(b, cudaMemcpy(b->res_d, blocks.data(), blocks.size() * sizeof(ResBlock), cudaMemcpyHostToDevice));
-  B_CUDA(b, cudaMemcpy(b->res_d + b->res_inst_at, insts.data(), insts.size() * sizeof(ResInst), cudaMemcpyHostToDevice));
-  B_CUDA(b, cudaMemset(b->res_d + b->res_out_at, 0xff, out_bytes));  // words tagged as no state's
+  B_CUDA(b, cudaMemcpy(b->res_d, tables.data(), tables.size(), cudaMemcpyHostToDevice));
+  B_CUDA(b, cudaMemset(b->res_d + b->res_out_at, 0, out_bytes));  // words of no state
   b->res_blocks = static_cast<int>(blocks.size());
   return LBM_OK;
 }
@@ -1051,9 +1057,9 @@ int get_inst_t(lbm_batch* b, int k, void* aos_dev) {
   const auto& in = b->inst[k];
   const long long n = static_cast<long long>(in.nx) * in.ny;
   const int grid = static_cast<int>(std::min<long long>((n + 255) / 256, 16LL * b->sm_count));
-  get_state_kernel<ST><<<grid, 256, 0, b->stream>>>(static_cast<const ST*>(b->buf[b->cur]) + in.off,
+  get_state_kernel<ST><<<grid, kGetThreads, 0, b->stream>>>(static_cast<const ST*>(b->buf[b->cur]) + in.off,
                                                     b->mask_d + in.mask_off, in.g, Eq9<T>{}, b->sc,
-                                                    static_cast<T*>(aos_dev));
+                                                    static_cast<T*>(aos_dev), 0, in.ny);
   B_CUDA(b, cudaGetLastError());
   return LBM_OK;
 }
@@ -1113,7 +1119,14 @@ int set_pop_t(lbm_batch* b, int k, const void* host) {
   const auto& in = b->inst[k];
   const size_t bytes = static_cast<size_t>(in.nx) * in.ny * kQ * sizeof(T);
   if (int rc = ensure_stage(b, bytes)) return rc;
-  B_CUDA(b, cudaMemcpyAsync(b->stage, host, bytes, cudaMemcpyHostToDevice, b->stream));
+  const void* view = bytes % 16 == 0 ? host_view(host, bytes, 16, b->direct, false) : nullptr;
+  if (view && reinterpret_cast<uintptr_t>(view) % 16 == 0) {
+    const long long n16 = static_cast<long long>(bytes / 16);
+    copy16_kernel<<<static_cast<int>(std::min<long long>((n16 + 255) / 256, 16LL * b->sm_count)), 256, 0, b->stream>>>(
+        static_cast<const uint4*>(view), static_cast<uint4*>(b->stage), n16);
+  } else {
+    B_CUDA(b, cudaMemcpyAsync(b->stage, host, bytes, cudaMemcpyHostToDevice, b->stream));
+  }
   if (int rc = set_inst_t<ST>(b, k, b->stage, Eq9<T>{})) return rc;
   B_CUDA(b, cudaStreamSynchronize(b->stream));
   return LBM_OK;
@@ -1124,6 +1137,11 @@ int get_pop_t(lbm_batch* b, int k, void* host) {
   using T = typename StoreTraits<ST>::T;
   const auto& in = b->inst[k];
   const size_t bytes = static_cast<size_t>(in.nx) * in.ny * kQ * sizeof(T);
+  if (void* view = host_view(host, bytes, sizeof(T), b->direct, true)) {  // written in place
+    if (int rc = get_inst_t<ST>(b, k, view)) return rc;
+    B_CUDA(b, cudaStreamSynchronize(b->stream));
+    return LBM_OK;
+  }
   if (int rc = ensure_stage(b, bytes)) return rc;
   if (int rc = get_inst_t<ST>(b, k, b->stage)) return rc;
   B_CUDA(b, cudaMemcpyAsync(host, b->stage, bytes, cudaMemcpyDeviceToHost, b->stream));
@@ -1240,6 +1258,7 @@ int lbm_batch_create(int count, const int* nx, const int* ny, const uint8_t* con
       cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&b->ev[0]) != cudaSuccess || cudaEventCreate(&b->ev[1]) != cudaSuccess)
     return fail(LBM_ERR_CUDA);
+  b->direct = host_memory_direct(b->device);
   const size_t bytes = static_cast<size_t>(off) * elem + 256;
   cudaError_t e = cudaSuccess;
   for (int k = 0; k < 2 && e == cudaSuccess; ++k) {

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "aux_kernels.cuh"
+#include "host_access.h"
 #include "lbm_b200.h"
 #include "solver_internal.h"
 #include "step_kernel.cuh"
@@ -421,9 +422,9 @@ template <class ST>
 int get_state_t(lbm_solver* s, void* aos_dev) {
   using T = typename StoreTraits<ST>::T;
   const long long n = static_cast<long long>(s->nx) * s->ny;
-  get_state_kernel<ST><<<grid_for_cells(s, n, 256), 256, 0, s->stream>>>(
+  get_state_kernel<ST><<<grid_for_cells(s, n, 256), kGetThreads, 0, s->stream>>>(
       static_cast<const ST*>(s->buf[s->cur]), s->mask_d, s->g, inlet_eq<ST>(s), s->sc,
-      static_cast<T*>(aos_dev));
+      static_cast<T*>(aos_dev), 0, s->ny);
   LBM_CUDA(s, cudaGetLastError());
   return LBM_OK;
 }
@@ -436,7 +437,7 @@ int moments_t(lbm_solver* s, void* rho, void* ux, void* uy) {
   const T hfx = T(0.5) * T(s->fx), hfy = T(0.5) * T(s->fy);
   moments_kernel<ST, A><<<grid_for_cells(s, n, 256), 256, 0, s->stream>>>(
       static_cast<const ST*>(s->buf[s->cur]), s->mask_d, s->g, inlet_eq<ST>(s), s->sc, hfx, hfy,
-      static_cast<T*>(rho), static_cast<T*>(ux), static_cast<T*>(uy));
+      static_cast<T*>(rho), static_cast<T*>(ux), static_cast<T*>(uy), 0, s->ny);
   LBM_CUDA(s, cudaGetLastError());
   return LBM_OK;
 }
@@ -692,12 +693,26 @@ int lbm_create(int nx, int ny, const uint8_t* solid, double tau, double fx, doub
   if (e != cudaSuccess) return fail(LBM_ERR_CUDA);
 
   const size_t state_bytes = static_cast<size_t>(kQ) * s->g.plane * elem + 256;
+  // The outboxes of resident launches, for the closed cut and the open one, lie behind the second
+  // state: one allocation and one memset (of zeros: words of no state) less per solver.
+  int coop = 0, optin = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device);
+  const size_t out_at = (state_bytes + 255) / 256 * 256;
+  size_t out_bytes = 0;
+  s->can_reside = coop && static_cast<size_t>(optin) >= kResSmemBytes;
+  if (s->can_reside) {
+    s->res = plan_resident(s, false);
+    out_bytes = std::max(outbox_bytes(s->res), outbox_bytes(plan_resident(s, true)));
+  }
   for (int b = 0; b < 2; ++b) {
-    e = cudaMalloc(&s->buf[b], state_bytes);
+    const size_t bytes = b == 1 && out_bytes ? out_at + out_bytes : state_bytes;
+    e = cudaMalloc(&s->buf[b], bytes);
     if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? LBM_ERR_OUT_OF_MEMORY : LBM_ERR_CUDA);
-    e = cudaMemsetAsync(s->buf[b], 0, state_bytes, s->stream);
+    e = cudaMemsetAsync(s->buf[b], 0, bytes, s->stream);
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA);
   }
+  if (out_bytes) s->outbox = static_cast<char*>(s->buf[1]) + out_at;
   s->state_bytes = state_bytes;
   std::vector<uint32_t> words;
   pack_mask(solid, nx, ny, s->g.mask_words, words);
@@ -707,26 +722,11 @@ int lbm_create(int nx, int ny, const uint8_t* solid, double tau, double fx, doub
                         cudaMemcpyHostToDevice, s->stream);
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? LBM_ERR_OUT_OF_MEMORY : LBM_ERR_CUDA);
   s->red_blocks = 4 * s->sm_count;
-  // One allocation: the reduction scratch, the flags, and from the next 256-byte boundary the
-  // outboxes of resident launches, for the closed cut and the open one.
   const size_t red_bytes = (s->red_blocks + 2) * sizeof(double) + 4 * sizeof(int);
-  const size_t out_at = (red_bytes + 255) / 256 * 256;
-  int coop = 0, optin = 0;
-  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device);
-  size_t out_bytes = 0;
-  s->can_reside = coop && static_cast<size_t>(optin) >= kResSmemBytes;
-  if (s->can_reside) {
-    s->res = plan_resident(s, false);
-    out_bytes = std::max(outbox_bytes(s->res), outbox_bytes(plan_resident(s, true)));
-  }
-  e = cudaMalloc(&s->red, out_at + out_bytes);
+  e = cudaMalloc(&s->red, red_bytes);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->red, 0, red_bytes, s->stream);
-  if (e == cudaSuccess && out_bytes) {  // words tagged as no state's
-    s->outbox = reinterpret_cast<char*>(s->red) + out_at;
-    e = cudaMemsetAsync(s->outbox, 0xff, out_bytes, s->stream);
-  }
-  s->err_flag = reinterpret_cast<int*>(s->red + s->red_blocks + 2) + 1;
+  s->direct = host_memory_direct(s->device);
+  s->err_flag = s->direct ? const_cast<int*>(&s->box.flag) : reinterpret_cast<int*>(s->red + s->red_blocks + 2) + 1;
   s->step_ctr = reinterpret_cast<uint32_t*>(s->red + s->red_blocks + 2) + 2;
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? LBM_ERR_OUT_OF_MEMORY : LBM_ERR_CUDA);
   e = cudaStreamSynchronize(s->stream);
@@ -780,25 +780,14 @@ int lbm_init_equilibrium(lbm_solver* s, double rho0, double ux0, double uy0) {
   LBM_DISPATCH(s, init_eq_t, s, rho0, ux0, uy0);
 }
 
-// Device address of a host buffer that kernels may access directly (pinned or registered host
-// memory, e.g. over NVLink-C2C), or null: pageable memory is staged through device memory.
-static const void* mapped_view(const void* p) {
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
-}
-
 int lbm_set_populations(lbm_solver* s, const void* s_host) {
   if (check(s) || !s_host) return set_error(s, LBM_ERR_INVALID_ARG, "null state");
   const size_t bytes = static_cast<size_t>(s->nx) * s->ny * kQ * s->host_elem;
   // One copy into device memory, then the conversion kernel (whose neighbour gathers would be
-  // slow over the host link): from pinned host memory with coalesced 16-byte kernel loads
-  // (size and address permitting), else with a copy engine.
+  // slow over the host link): from host memory that kernels can address with coalesced 16-byte
+  // loads (size and address permitting), else with a copy engine.
   if (int rc = ensure_stage(s, bytes)) return rc;
-  const void* mapped = mapped_view(s_host);
+  const void* mapped = host_view(s_host, bytes, 16, s->direct, false);
   if (mapped && bytes % 16 == 0 && reinterpret_cast<uintptr_t>(mapped) % 16 == 0) {
     const long long n16 = static_cast<long long>(bytes / 16);
     copy16_kernel<<<grid_for_cells(s, n16, 256), 256, 0, s->stream>>>(static_cast<const uint4*>(mapped),
@@ -830,6 +819,12 @@ int lbm_step(lbm_solver* s, int steps) {
 
 // Reads and clears the device error flag of the step kernels (a bounded wait that ran out).
 static int check_step_flag(lbm_solver* s) {
+  if (s->direct) {
+    LBM_CUDA(s, cudaStreamSynchronize(s->stream));
+    if (!s->box.flag) return LBM_OK;
+    s->box.flag = 0;
+    return set_error(s, LBM_ERR_TIMEOUT, "a step kernel gave up waiting for its shared-memory ring");
+  }
   int flag = 0;
   LBM_CUDA(s, cudaMemcpyAsync(&flag, s->err_flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   LBM_CUDA(s, cudaStreamSynchronize(s->stream));
@@ -843,7 +838,6 @@ static int check_step_flag(lbm_solver* s) {
 
 int lbm_synchronize(lbm_solver* s) {
   if (check(s)) return LBM_ERR_INVALID_ARG;
-  LBM_CUDA(s, cudaStreamSynchronize(s->stream));
   return check_step_flag(s);
 }
 
@@ -873,8 +867,9 @@ int lbm_timed_run(lbm_solver* s, int steps, double* seconds) {
 int lbm_get_populations(lbm_solver* s, void* s_host) {
   if (check(s) || !s_host) return set_error(s, LBM_ERR_INVALID_ARG, "null output");
   const size_t bytes = static_cast<size_t>(s->nx) * s->ny * kQ * s->host_elem;
-  // Pinned host output: the gather kernel writes it in place; else through device memory.
-  void* dst = const_cast<void*>(mapped_view(s_host));
+  // Host output that kernels can address: the gather kernel writes it in place; else through
+  // device memory.
+  void* dst = host_view(s_host, bytes, s->host_elem, s->direct, true);
   if (!dst) {
     if (int rc = ensure_stage(s, bytes)) return rc;
     dst = s->stage;
@@ -898,11 +893,11 @@ int lbm_macroscopic(lbm_solver* s, void* rho, void* ux, void* uy) {
   if (check(s) || !rho || !ux || !uy) return set_error(s, LBM_ERR_INVALID_ARG, "null output");
   const size_t n = static_cast<size_t>(s->nx) * s->ny;
   const size_t plane = n * s->host_elem;
-  // Pinned host outputs (all three): the moment kernel writes them in place; else through
-  // device memory.
-  void* mr = const_cast<void*>(mapped_view(rho));
-  void* mu = const_cast<void*>(mapped_view(ux));
-  void* mv = const_cast<void*>(mapped_view(uy));
+  // Host outputs that kernels can address (all three): the moment kernel writes them in place;
+  // else through device memory.
+  void* mr = host_view(rho, plane, s->host_elem, s->direct, true);
+  void* mu = mr ? host_view(ux, plane, s->host_elem, s->direct, true) : nullptr;
+  void* mv = mu ? host_view(uy, plane, s->host_elem, s->direct, true) : nullptr;
   const bool direct = mr && mu && mv;
   char* d = nullptr;
   if (!direct) {
@@ -932,8 +927,13 @@ int lbm_macroscopic(lbm_solver* s, void* rho, void* ux, void* uy) {
 
 int lbm_total_mass(lbm_solver* s, double* mass) {
   if (check(s) || !mass) return set_error(s, LBM_ERR_INVALID_ARG, "null output");
-  double* out = s->red + s->red_blocks;
+  double* out = s->direct ? s->box.out : s->red + s->red_blocks;
   if (int rc = lbm_b200::solver_mass_into(s, s->buf[s->cur], s->red, s->red_blocks, out)) return rc;
+  if (s->direct) {
+    LBM_CUDA(s, cudaStreamSynchronize(s->stream));
+    *mass = s->box.out[0];
+    return LBM_OK;
+  }
   LBM_CUDA(s, cudaMemcpyAsync(mass, out, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
   LBM_CUDA(s, cudaStreamSynchronize(s->stream));
   return LBM_OK;
@@ -943,16 +943,25 @@ int lbm_populations_at(lbm_solver* s, int x, int y, void* out9) {
   if (check(s) || !out9) return set_error(s, LBM_ERR_INVALID_ARG, "null output");
   if (x < 0 || x >= s->nx || y < 0 || y >= s->ny)
     return set_error(s, LBM_ERR_INVALID_ARG, "cell outside the grid");
-  if (int rc = ensure_stage(s, kQ * 8)) return rc;
+  void* dst = s->box.out;
+  if (!s->direct) {
+    if (int rc = ensure_stage(s, kQ * 8)) return rc;
+    dst = s->stage;
+  }
   int rc;
   switch (s->precision) {
-    case LBM_FP32: rc = probe_t<float>(s, x, y, s->stage); break;
-    case LBM_FP64: rc = probe_t<double>(s, x, y, s->stage); break;
-    case LBM_FP16_STORE: rc = probe_t<__half>(s, x, y, s->stage); break;
-    case LBM_BF16_STORE: rc = probe_t<__nv_bfloat16>(s, x, y, s->stage); break;
+    case LBM_FP32: rc = probe_t<float>(s, x, y, dst); break;
+    case LBM_FP64: rc = probe_t<double>(s, x, y, dst); break;
+    case LBM_FP16_STORE: rc = probe_t<__half>(s, x, y, dst); break;
+    case LBM_BF16_STORE: rc = probe_t<__nv_bfloat16>(s, x, y, dst); break;
     default: rc = LBM_ERR_INVALID_ARG;
   }
   if (rc) return rc;
+  if (s->direct) {
+    LBM_CUDA(s, cudaStreamSynchronize(s->stream));
+    std::memcpy(out9, s->box.out, kQ * s->host_elem);
+    return LBM_OK;
+  }
   LBM_CUDA(s, cudaMemcpyAsync(out9, s->stage, kQ * s->host_elem, cudaMemcpyDeviceToHost, s->stream));
   LBM_CUDA(s, cudaStreamSynchronize(s->stream));
   return LBM_OK;
@@ -980,7 +989,7 @@ int lbm_set_body(lbm_solver* s, const uint8_t* body) {
 int lbm_body_force(lbm_solver* s, double* fx, double* fy) {
   if (check(s) || !fx || !fy) return set_error(s, LBM_ERR_INVALID_ARG, "null output");
   if (!s->force_red) LBM_CUDA(s, cudaMalloc(&s->force_red, (2 * s->red_blocks + 2) * sizeof(double)));
-  double* out = s->force_red + 2 * s->red_blocks;
+  double* out = s->direct ? s->box.out : s->force_red + 2 * s->red_blocks;
   int rc;
   switch (s->precision) {
     case LBM_FP32: rc = body_force_t<float>(s, out); break;
@@ -991,8 +1000,9 @@ int lbm_body_force(lbm_solver* s, double* fx, double* fy) {
   }
   if (rc) return rc;
   double f[2];
-  LBM_CUDA(s, cudaMemcpyAsync(f, out, sizeof(f), cudaMemcpyDeviceToHost, s->stream));
+  if (!s->direct) LBM_CUDA(s, cudaMemcpyAsync(f, out, sizeof(f), cudaMemcpyDeviceToHost, s->stream));
   LBM_CUDA(s, cudaStreamSynchronize(s->stream));
+  if (s->direct) std::memcpy(f, s->box.out, sizeof(f));
   *fx = f[0];
   *fy = f[1];
   return LBM_OK;
@@ -1000,8 +1010,11 @@ int lbm_body_force(lbm_solver* s, double* fx, double* fy) {
 
 int lbm_check_finite(lbm_solver* s, int* finite) {
   if (check(s) || !finite) return set_error(s, LBM_ERR_INVALID_ARG, "null output");
-  int* flag = reinterpret_cast<int*>(s->red + s->red_blocks + 2);
-  LBM_CUDA(s, cudaMemsetAsync(flag, 0, sizeof(int), s->stream));
+  int* flag = s->direct ? const_cast<int*>(&s->box.bad) : reinterpret_cast<int*>(s->red + s->red_blocks + 2);
+  if (s->direct)
+    s->box.bad = 0;
+  else
+    LBM_CUDA(s, cudaMemsetAsync(flag, 0, sizeof(int), s->stream));
   int rc;
   switch (s->precision) {
     case LBM_FP32: rc = finite_t<float>(s, flag); break;
@@ -1012,8 +1025,9 @@ int lbm_check_finite(lbm_solver* s, int* finite) {
   }
   if (rc) return rc;
   int bad = 0;
-  LBM_CUDA(s, cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  if (!s->direct) LBM_CUDA(s, cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   LBM_CUDA(s, cudaStreamSynchronize(s->stream));
+  if (s->direct) bad = s->box.bad;
   *finite = bad ? 0 : 1;
   return LBM_OK;
 }

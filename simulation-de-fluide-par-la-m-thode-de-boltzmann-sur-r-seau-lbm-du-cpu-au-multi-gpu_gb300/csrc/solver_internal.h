@@ -10,6 +10,13 @@
 #include "lbm_device.cuh"
 #include "resident_layout.h"
 
+// Results that kernels write straight into host memory (where the device can).
+struct alignas(64) HostBox {
+  volatile int flag = 0;    // set by a step kernel whose bounded wait ran out
+  volatile int bad = 0;     // set by the finite check
+  double out[12] = {};      // mass, force, or one cell's populations
+};
+
 struct lbm_solver {
   int nx = 0, ny = 0, precision = 0;
   lbm_b200::Grid2D g{};
@@ -34,16 +41,20 @@ struct lbm_solver {
   double u_in = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  double* red = nullptr;  // mass partials [red_blocks], result, spare, then int flags, then outboxes
+  double* red = nullptr;  // mass partials [red_blocks], result, spare, then int flags
   int red_blocks = 0;
   void* stage = nullptr;  // device staging for host input / output
   size_t stage_bytes = 0;
   int block = 256, grid = 0, last_grid = 0;  // step launch shape (grid 0: persistent, automatic)
-  int* err_flag = nullptr;  // set by a step kernel whose bounded wait ran out
+  // Set by a step kernel whose bounded wait ran out: in `box` where kernels reach host memory
+  // (direct), else in device memory.
+  int* err_flag = nullptr;
+  bool direct = false;
+  HostBox box;
   int variant = -1;      // step kernel variant (lbm_set_variant); -1: chosen from the grid shape
   int last_variant = 0;  // variant of the last launch
   // Resident launches (step_resident.cuh): the device can run them, the cut of the grid (tx = 0:
-  // it does not fit), the tiles' outboxes (in red's allocation).
+  // it does not fit), the tiles' outboxes (behind buf[1]'s state).
   bool can_reside = false;
   lbm_b200::ResLayout res{};
   void* outbox = nullptr;

@@ -252,7 +252,8 @@ __device__ __forceinline__ void resident_body(unsigned char* smem, const StepArg
   const int nitems = items.total, npolls = res_polls<static_cast<int>(sizeof(ST))>(w, h);
   const int mw = (w + 2 + 31) / 32 + 1;
   const long long per_parity = static_cast<long long>(L.words()) * L.tx * L.ty;
-  const uint32_t t0 = __ldg(tag_ctr), step0 = sizeof(ST) == 2 ? __ldg(p.step_ctr) : 0u;
+  // Tags start at 1: outboxes are created as zeros.
+  const uint32_t t0 = __ldg(tag_ctr) + 1u, step0 = sizeof(ST) == 2 ? __ldg(p.step_ctr) : 0u;
 
   // Tables: mask bits (bit j of a row: cell x0 - 1 + j; rows -1 .. h), poll list, items.
   for (int k = tid; k < (h + 2) * mw; k += kThreads) {

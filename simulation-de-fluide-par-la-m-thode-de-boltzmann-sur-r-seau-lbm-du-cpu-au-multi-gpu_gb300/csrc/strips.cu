@@ -33,6 +33,7 @@
 #include "aux_kernels.cuh"
 #include "fastdiv.h"
 #include "forms.cuh"
+#include "host_access.h"
 #include "lbm_b200.h"
 #include "solver_internal.h"
 #include "step_ring.cuh"
@@ -214,6 +215,7 @@ struct lbm_strips {
   bool graphs = true;
   int passes = 2;  // ring passes per strip: 4 (2048-cell tiles) for 16-bit storage on rows >= 2048
   int sm_count = 0;
+  bool direct = false;  // kernels reach host memory
   std::string err;
 };
 
@@ -429,44 +431,45 @@ int set_t(lbm_strips* h, const void* s_host, Eq9<typename StoreTraits<ST>::T> eq
   return LBM_OK;
 }
 
-// Owned rows of every strip: v0-layout populations (what = 0) or rho/ux/uy (what = 1).
+// Owned rows of every strip: v0-layout populations (what = 0) or rho/ux/uy (what = 1). The gather
+// kernels write each strip's owned rows where they lie in the whole lattice: in the host output
+// itself where kernels can address it, else in device memory that is copied once.
 template <class ST>
 int get_t(lbm_strips* h, int what, void* out0, void* out1, void* out2) {
   using T = typename StoreTraits<ST>::T;
   using A = typename Form<ST>::A;
-  const int nx = h->nx;
+  const int nx = h->nx, fields = what == 0 ? 1 : 3;
+  const size_t n = static_cast<size_t>(nx) * h->ny, bytes = n * (what == 0 ? kQ : 1) * sizeof(T);
   const Eq9<T> eq_in = strip_inlet<ST>(h, false);
-  std::vector<T> local;
+  void* outs[3] = {out0, out1, out2};
+  T* dst[3] = {nullptr, nullptr, nullptr};
+  bool in_place = true;
+  for (int f = 0; f < fields && in_place; ++f) {
+    dst[f] = static_cast<T*>(host_view(outs[f], bytes, sizeof(T), h->direct, true));
+    in_place = dst[f] != nullptr;
+  }
+  if (!in_place) {
+    if (int rc = ensure_stage(h, fields * bytes)) return rc;
+    for (int f = 0; f < fields; ++f) dst[f] = reinterpret_cast<T*>(static_cast<char*>(h->stage) + f * bytes);
+  }
   for (int k = 0; k < h->strips; ++k) {
     const Grid2D g = strip_grid(h, k);
-    const size_t cells = static_cast<size_t>(nx) * g.ny;
-    const size_t per_cell = what == 0 ? kQ : 3;
-    if (int rc = ensure_stage(h, cells * per_cell * sizeof(T))) return rc;
-    T* st = static_cast<T*>(h->stage);
+    const size_t at = static_cast<size_t>(h->y0[k]) * nx;
     const ST* R = static_cast<const ST*>(h->buf[h->cur]) + h->off[k];
-    const int grid = grid_cells(h, static_cast<long long>(cells));
-    if (what == 0) {
-      get_state_kernel<ST><<<grid, 256, 0, h->stream>>>(R, h->mask_d + h->moff[k], g, eq_in, h->sc, st);
-    } else {
+    const int grid = grid_cells(h, static_cast<long long>(nx) * h->n[k]);
+    if (what == 0)
+      get_state_kernel<ST><<<grid, kGetThreads, 0, h->stream>>>(R, h->mask_d + h->moff[k], g, eq_in, h->sc, dst[0] + at * kQ,
+                                                        1, h->n[k]);
+    else
       moments_kernel<ST, A><<<grid, 256, 0, h->stream>>>(R, h->mask_d + h->moff[k], g, eq_in, h->sc,
-                                                         T(T(0.5) * T(h->fx)), T(T(0.5) * T(h->fy)), st,
-                                                         st + cells, st + 2 * cells);
-    }
+                                                         T(T(0.5) * T(h->fx)), T(T(0.5) * T(h->fy)), dst[0] + at,
+                                                         dst[1] + at, dst[2] + at, 1, h->n[k]);
     S_CUDA(h, cudaGetLastError());
-    local.resize(cells * per_cell);
-    S_CUDA(h, cudaMemcpyAsync(local.data(), st, cells * per_cell * sizeof(T), cudaMemcpyDeviceToHost, h->stream));
-    S_CUDA(h, cudaStreamSynchronize(h->stream));
-    const size_t row0 = static_cast<size_t>(h->y0[k]) * nx;
-    const size_t owned = static_cast<size_t>(h->n[k]) * nx;
-    if (what == 0) {
-      std::memcpy(static_cast<T*>(out0) + row0 * kQ, local.data() + static_cast<size_t>(nx) * kQ,
-                  owned * kQ * sizeof(T));
-    } else {
-      void* outs[3] = {out0, out1, out2};
-      for (int f = 0; f < 3; ++f)
-        std::memcpy(static_cast<T*>(outs[f]) + row0, local.data() + f * cells + nx, owned * sizeof(T));
-    }
   }
+  if (!in_place)
+    for (int f = 0; f < fields; ++f)
+      S_CUDA(h, cudaMemcpyAsync(outs[f], dst[f], bytes, cudaMemcpyDeviceToHost, h->stream));
+  S_CUDA(h, cudaStreamSynchronize(h->stream));
   return LBM_OK;
 }
 
@@ -577,6 +580,7 @@ int lbm_strips_create(int nx, int ny, const uint8_t* solid, double tau, double f
       cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&h->ev[0]) != cudaSuccess || cudaEventCreate(&h->ev[1]) != cudaSuccess)
     return fail(LBM_ERR_CUDA);
+  h->direct = host_memory_direct(device);
   const size_t bytes = static_cast<size_t>(off) * elem + 256;
   cudaError_t e = cudaSuccess;
   for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
