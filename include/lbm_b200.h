@@ -114,8 +114,8 @@ int lbm_timed_run(lbm_solver* s, int steps, double* seconds);
 /* Waits for all work of s. */
 int lbm_synchronize(lbm_solver* s);
 
-/* Number of kernels s has enqueued for time steps so far: one per step plus one step-counter
- * update per launch sequence (a replayed step graph counts the kernels it holds, a launch that
+/* Number of kernels s has enqueued for time steps so far: one per step, plus one step-counter
+ * update per launch sequence of the 16-bit forms and per resident launch (a replayed step graph counts the kernels it holds, a launch that
  * takes many steps counts one per step). For
  * benchmarks that report how many of the library's kernels ran in a timed region. */
 int lbm_kernel_launches(const lbm_solver* s, long long* count);

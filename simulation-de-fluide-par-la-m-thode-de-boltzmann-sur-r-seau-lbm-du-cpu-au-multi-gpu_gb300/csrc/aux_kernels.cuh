@@ -7,6 +7,9 @@
 
 namespace lbm_b200 {
 
+// Threads of the kernels that move v0-layout states through shared memory.
+constexpr int kGetThreads = 256;
+
 __device__ __forceinline__ long long cell_index(const Grid2D& g, int x, int y) {
   return static_cast<long long>(y) * g.pitch + x;
 }
@@ -74,11 +77,60 @@ __global__ void set_state_kernel(ST* __restrict__ R, const uint32_t* __restrict_
   }
 }
 
+// The same preimage from a v0-layout state, by the values' destinations: post-streaming value i of
+// a fluid cell came from slot (c - e_i, i), or from slot (c, opp i) where c - e_i is solid, so each
+// value is read once and goes to one slot, each slot of a fluid cell gets one. Blocks read
+// contiguous runs (through shared memory), so that the state may lie in host memory (4096^2 FP32,
+// pinned: 2.88 ms; a copy into device memory and the gather of set_state_kernel 3.20 ms). Slots that
+// leave an open domain, which nothing pulls, take the cell's own value; solid cells' slots zeros.
+template <class ST>
+__global__ void __launch_bounds__(kGetThreads)
+    scatter_state_kernel(ST* __restrict__ R, const uint32_t* __restrict__ mask, const Grid2D g,
+                         const typename StoreTraits<ST>::T* __restrict__ aos, const PlaneScales sc) {
+  using T = typename StoreTraits<ST>::T;
+  __shared__ T run[kGetThreads * kQ];
+  const long long n = static_cast<long long>(g.nx) * g.ny;
+  for (long long c0 = static_cast<long long>(blockIdx.x) * kGetThreads; c0 < n;
+       c0 += static_cast<long long>(gridDim.x) * kGetThreads) {
+    const long long c = c0 + threadIdx.x;
+    const int cells = static_cast<int>(n - c0 < kGetThreads ? n - c0 : kGetThreads);
+    if (cells == kGetThreads) {
+#pragma unroll
+      for (int k = 0; k < kQ; ++k) run[k * kGetThreads + threadIdx.x] = aos[c0 * kQ + k * kGetThreads + threadIdx.x];
+    } else {
+      for (int k = threadIdx.x; k < cells * kQ; k += kGetThreads) run[k] = aos[c0 * kQ + k];
+    }
+    __syncthreads();
+    if (c < n) {
+      const int y = static_cast<int>(c / g.nx), x = static_cast<int>(c - static_cast<long long>(y) * g.nx);
+      const bool solid = mask_solid(mask, g.mask_words, x, y);
+#pragma unroll
+      for (int i = 0; i < kQ; ++i) {
+        if (solid) {
+          R[i * g.plane + cell_index(g, x, y)] = encode<ST>(T(0), i, sc);
+          continue;
+        }
+        const T v = run[threadIdx.x * kQ + i];
+        const int xr = x - dir_cx(i), xn = x + dir_cx(i);
+        if (g.open_x && (xn < 0 || xn >= g.nx)) R[i * g.plane + cell_index(g, x, y)] = encode<ST>(v, i, sc);
+        if (g.open_x && (xr < 0 || xr >= g.nx)) continue;  // from the inlet or the outlet's copy
+        const int xs = xr < 0 ? g.nx - 1 : (xr >= g.nx ? 0 : xr);
+        int ys = y - dir_cy(i);
+        ys = ys < 0 ? g.ny - 1 : (ys >= g.ny ? 0 : ys);
+        if (mask_solid(mask, g.mask_words, xs, ys))
+          R[dir_opp(i) * g.plane + cell_index(g, x, y)] = encode<ST>(v, dir_opp(i), sc);
+        else
+          R[i * g.plane + cell_index(g, xs, ys)] = encode<ST>(v, i, sc);
+      }
+    }
+    __syncthreads();
+  }
+}
+
 // Pull state -> post-streaming state in v0 layout (solid cells 0) of `rows` rows from row0 on, by
 // blocks of kGetThreads. A block's cells pass through shared memory, so that it writes one
 // contiguous run: nine values a thread apart would cross to host memory as partial sectors
 // (26 MB into pinned or pageable host memory: 1050 us, 170 us as runs).
-constexpr int kGetThreads = 256;
 template <class ST>
 __global__ void __launch_bounds__(kGetThreads)
     get_state_kernel(const ST* __restrict__ R, const uint32_t* __restrict__ mask, const Grid2D g,
@@ -235,18 +287,24 @@ static __global__ void copy16_kernel(const uint4* __restrict__ src, uint4* __res
 // fluid cell x to a body cell x + c_i carries 2 c_i f*_i(x), with f*_i(x) = R_i(x) + w_i the
 // post-collision population of x leaving along c_i (the pull state holds post-collision
 // values), which bounces back unchanged. Links leaving an open x boundary carry nothing. FP64
-// per-block partials of (F_x, F_y).
+// per-block partials of (F_x, F_y) over the cells bx .. bx + bw - 1, by .. by + bh - 1 (periodic):
+// the box around the body (1024 x 256 with a disc of 32 cells: 23.7 us a call for the whole grid,
+// 18.7 us for its box).
 template <class ST>
 __global__ void __launch_bounds__(kReduceThreads)
     body_force_partial_kernel(const ST* __restrict__ R, const uint32_t* __restrict__ mask,
                               const uint32_t* __restrict__ body, const Grid2D g,
-                              const PlaneScales sc, double* __restrict__ partials) {
+                              const PlaneScales sc, int bx, int by, int bw, int bh,
+                              double* __restrict__ partials) {
   __shared__ double smem[32];
   double ax = 0.0, ay = 0.0;
-  const long long n = static_cast<long long>(g.nx) * g.ny;
+  const long long n = static_cast<long long>(bw) * bh;
   for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
        c += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int y = static_cast<int>(c / g.nx), x = static_cast<int>(c - static_cast<long long>(y) * g.nx);
+    const int r = static_cast<int>(c / bw);
+    int y = by + r, x = bx + static_cast<int>(c - static_cast<long long>(r) * bw);
+    y = y < 0 ? y + g.ny : (y >= g.ny ? y - g.ny : y);
+    x = x < 0 ? x + g.nx : (x >= g.nx ? x - g.nx : x);
     if (mask_solid(mask, g.mask_words, x, y)) continue;
 #pragma unroll
     for (int i = 1; i < kQ; ++i) {
@@ -261,11 +319,11 @@ __global__ void __launch_bounds__(kReduceThreads)
       ay += 2.0 * dir_cy(i) * f;
     }
   }
-  const double bx = block_sum(ax, smem);
-  const double by = block_sum(ay, smem);
+  const double sx = block_sum(ax, smem);
+  const double sy = block_sum(ay, smem);
   if (threadIdx.x == 0) {
-    partials[2 * blockIdx.x] = bx;
-    partials[2 * blockIdx.x + 1] = by;
+    partials[2 * blockIdx.x] = sx;
+    partials[2 * blockIdx.x + 1] = sy;
   }
 }
 
@@ -273,6 +331,7 @@ __global__ void __launch_bounds__(kReduceThreads)
 static __global__ void __launch_bounds__(kReduceThreads)
     pair_final_kernel(const double* __restrict__ partials, int count, double* __restrict__ out) {
   __shared__ double smem[32];
+  grid_dependency_wait();
   double ax = 0.0, ay = 0.0;
   for (int k = threadIdx.x; k < count; k += blockDim.x) {
     ax += partials[2 * k];

@@ -386,6 +386,9 @@ int launch_resident(lbm_solver* s, int steps) {
   }
 }
 
+// Do the step kernels' launch sequences end with a counter update?
+bool counts_steps(const lbm_solver* s) { return s->elem == 2; }
+
 // Runs of at least kResidentMinSteps steps take resident launches where the grid fits and the
 // caller has not chosen a kernel.
 bool use_resident(const lbm_solver* s, int steps) {
@@ -398,22 +401,31 @@ int launch_steps(lbm_solver* s, int steps) {
     if (use_resident(s, steps)) return launch_resident<ST>(s, steps);
   const int rc = s->open_x ? launch_steps_o<ST, true>(s, steps) : launch_steps_o<ST, false>(s, steps);
   if (rc) return rc;
-  LBM_CUDA(s, launch_dependent(counter_add_dep_kernel, dim3(1), dim3(1), 0, s->stream, s->step_ctr,
-                               static_cast<uint32_t>(steps)));
+  // The counter keys the rounding of the 16-bit forms (and numbers resident states, whose launches
+  // advance it themselves): FP32 and FP64 steps go without the update.
+  if (counts_steps(s))
+    LBM_CUDA(s, launch_dependent(counter_add_dep_kernel, dim3(1), dim3(1), 0, s->stream, s->step_ctr,
+                                 static_cast<uint32_t>(steps)));
   LBM_CUDA(s, cudaGetLastError());
   return LBM_OK;
 }
 
+// The current state from a uniform equilibrium, or from v0-layout populations that kernels can
+// address.
 template <class ST>
-int set_state_t(lbm_solver* s, const void* aos_dev, Eq9<typename StoreTraits<ST>::T> eq) {
+int set_equilibrium_t(lbm_solver* s, Eq9<typename StoreTraits<ST>::T> eq) {
+  const long long n = static_cast<long long>(s->nx) * s->ny;
+  set_state_kernel<ST><<<grid_for_cells(s, n, 256), 256, 0, s->stream>>>(static_cast<ST*>(s->buf[s->cur]), s->mask_d,
+                                                                         s->g, nullptr, eq, s->sc);
+  LBM_CUDA(s, cudaGetLastError());
+  return LBM_OK;
+}
+template <class ST>
+int set_state_t(lbm_solver* s, const void* aos) {
   using T = typename StoreTraits<ST>::T;
   const long long n = static_cast<long long>(s->nx) * s->ny;
-  const int grid = grid_for_cells(s, n, 256);
-  // Both buffers: the step never writes solid cells of an all-solid chunk, so they must hold 0
-  // in the buffer it writes too (cudaMemset at creation); the current one gets the state.
-  set_state_kernel<ST><<<grid, 256, 0, s->stream>>>(static_cast<ST*>(s->buf[s->cur]), s->mask_d,
-                                                    s->g, static_cast<const T*>(aos_dev), eq,
-                                                    s->sc);
+  scatter_state_kernel<ST><<<grid_for_cells(s, n, kGetThreads), kGetThreads, 0, s->stream>>>(
+      static_cast<ST*>(s->buf[s->cur]), s->mask_d, s->g, static_cast<const T*>(aos), s->sc);
   LBM_CUDA(s, cudaGetLastError());
   return LBM_OK;
 }
@@ -463,12 +475,18 @@ int finite_t(lbm_solver* s, int* flag) {
 
 template <class ST>
 int body_force_t(lbm_solver* s, double* out) {
-  const long long n = static_cast<long long>(s->nx) * s->ny;
   const uint32_t* body = s->body_d ? s->body_d : s->mask_d;
-  body_force_partial_kernel<ST><<<s->red_blocks, kReduceThreads, 0, s->stream>>>(
-      static_cast<const ST*>(s->buf[s->cur]), s->mask_d, body, s->g, s->sc, s->force_red);
-  pair_final_kernel<<<1, kReduceThreads, 0, s->stream>>>(s->force_red, s->red_blocks, out);
-  (void)n;
+  // Only cells next to the body feel it: scan the box around it (the whole grid without one).
+  int box[4] = {0, 0, s->nx, s->ny};
+  if (s->body_d) std::copy(s->body_box, s->body_box + 4, box);
+  const long long n = static_cast<long long>(box[2]) * box[3];
+  const int blocks =
+      static_cast<int>(std::max<long long>(1, std::min<long long>(s->red_blocks, (n + kReduceThreads - 1) / kReduceThreads)));
+  body_force_partial_kernel<ST><<<blocks, kReduceThreads, 0, s->stream>>>(
+      static_cast<const ST*>(s->buf[s->cur]), s->mask_d, body, s->g, s->sc, box[0], box[1], box[2], box[3],
+      s->force_red);
+  LBM_CUDA(s, launch_dependent(pair_final_kernel, dim3(1), dim3(kReduceThreads), 0, s->stream,
+                               static_cast<const double*>(s->force_red), blocks, out));
   LBM_CUDA(s, cudaGetLastError());
   return LBM_OK;
 }
@@ -496,7 +514,7 @@ int probe_t(lbm_solver* s, int x, int y, void* out) {
 template <class ST>
 int init_eq_t(lbm_solver* s, double rho0, double ux0, double uy0) {
   using T = typename StoreTraits<ST>::T;
-  return set_state_t<ST>(s, nullptr, host_equilibrium<T>(T(rho0), T(ux0), T(uy0)));
+  return set_equilibrium_t<ST>(s, host_equilibrium<T>(T(rho0), T(ux0), T(uy0)));
 }
 
 int ensure_stage(lbm_solver* s, size_t bytes) {
@@ -591,13 +609,14 @@ int solver_step_raw(lbm_solver* s, int steps) {
     if (int rc = ensure_step_graph(s)) return rc;
     while (s->graph && steps >= kGraphSteps) {
       LBM_CUDA(s, cudaGraphLaunch(s->graph, s->stream));
-      s->kernels += kGraphSteps + 1;  // the graph's step launches and its step-counter update
+      s->kernels += kGraphSteps + (counts_steps(s) ? 1 : 0);  // the graph's launches
       steps -= kGraphSteps;
     }
   }
   if (steps <= 0) return LBM_OK;
+  const bool update = counts_steps(s) || use_resident(s, steps);
   const int rc = solver_launch(s, steps);
-  if (!rc) s->kernels += steps + 1;
+  if (!rc) s->kernels += steps + (update ? 1 : 0);
   return rc;
 }
 
@@ -783,26 +802,20 @@ int lbm_init_equilibrium(lbm_solver* s, double rho0, double ux0, double uy0) {
 int lbm_set_populations(lbm_solver* s, const void* s_host) {
   if (check(s) || !s_host) return set_error(s, LBM_ERR_INVALID_ARG, "null state");
   const size_t bytes = static_cast<size_t>(s->nx) * s->ny * kQ * s->host_elem;
-  // One copy into device memory, then the conversion kernel (whose neighbour gathers would be
-  // slow over the host link): from host memory that kernels can address with coalesced 16-byte
-  // loads (size and address permitting), else with a copy engine.
-  if (int rc = ensure_stage(s, bytes)) return rc;
-  const void* mapped = host_view(s_host, bytes, 16, s->direct, false);
-  if (mapped && bytes % 16 == 0 && reinterpret_cast<uintptr_t>(mapped) % 16 == 0) {
-    const long long n16 = static_cast<long long>(bytes / 16);
-    copy16_kernel<<<grid_for_cells(s, n16, 256), 256, 0, s->stream>>>(static_cast<const uint4*>(mapped),
-                                                                      static_cast<uint4*>(s->stage), n16);
-    LBM_CUDA(s, cudaGetLastError());
-  } else {
+  // The conversion reads host memory that kernels can address in place (each value once, in
+  // contiguous runs), else a copy of it in device memory.
+  const void* src = host_view(s_host, bytes, s->host_elem, s->direct, false);
+  if (!src) {
+    if (int rc = ensure_stage(s, bytes)) return rc;
     LBM_CUDA(s, cudaMemcpyAsync(s->stage, s_host, bytes, cudaMemcpyHostToDevice, s->stream));
+    src = s->stage;
   }
-  const void* src = s->stage;
   int rc;
   switch (s->precision) {
-    case LBM_FP32: rc = set_state_t<float>(s, src, Eq9<float>{}); break;
-    case LBM_FP64: rc = set_state_t<double>(s, src, Eq9<double>{}); break;
-    case LBM_FP16_STORE: rc = set_state_t<__half>(s, src, Eq9<float>{}); break;
-    case LBM_BF16_STORE: rc = set_state_t<__nv_bfloat16>(s, src, Eq9<float>{}); break;
+    case LBM_FP32: rc = set_state_t<float>(s, src); break;
+    case LBM_FP64: rc = set_state_t<double>(s, src); break;
+    case LBM_FP16_STORE: rc = set_state_t<__half>(s, src); break;
+    case LBM_BF16_STORE: rc = set_state_t<__nv_bfloat16>(s, src); break;
     default: rc = LBM_ERR_INVALID_ARG;
   }
   if (rc) return rc;
@@ -977,6 +990,19 @@ int lbm_set_body(lbm_solver* s, const uint8_t* body) {
   const size_t n = static_cast<size_t>(s->nx) * s->ny;
   for (size_t c = 0; c < n; ++c)
     if (body[c] && !s->solid[c]) return set_error(s, LBM_ERR_INVALID_ARG, "body cells must be solid");
+  // The box of the body's cells and their neighbours: first cell (periodic) and extent.
+  int lo[2] = {s->nx, s->ny}, hi[2] = {-1, -1};
+  for (int y = 0; y < s->ny; ++y)
+    for (int x = 0; x < s->nx; ++x)
+      if (body[static_cast<size_t>(y) * s->nx + x]) {
+        lo[0] = std::min(lo[0], x), hi[0] = std::max(hi[0], x);
+        lo[1] = std::min(lo[1], y), hi[1] = std::max(hi[1], y);
+      }
+  for (int d = 0; d < 2; ++d) {
+    const int size = d == 0 ? s->nx : s->ny, extent = hi[d] < 0 ? 0 : hi[d] - lo[d] + 3;
+    s->body_box[d] = extent >= size || extent == 0 ? 0 : lo[d] - 1;
+    s->body_box[2 + d] = std::min(extent, size);
+  }
   std::vector<uint32_t> words;
   pack_mask(body, s->nx, s->ny, s->g.mask_words, words);
   const size_t bytes = words.size() * sizeof(uint32_t);

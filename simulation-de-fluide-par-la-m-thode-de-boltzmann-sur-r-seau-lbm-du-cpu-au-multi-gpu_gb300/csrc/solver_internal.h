@@ -33,6 +33,7 @@ struct lbm_solver {
   size_t state_bytes = 0;
   uint32_t* mask_d = nullptr;  // bit-packed mask with periodic ghost bits
   uint32_t* body_d = nullptr;  // bit-packed body of lbm_body_force (null: every solid cell)
+  int body_box[4] = {0, 0, 0, 0};  // box around it: first column and row (may be -1), columns, rows
   double* force_red = nullptr;  // body-force partials [2 red_blocks], then the result pair
   std::vector<uint8_t> solid;  // host copy (the reference's solid())
   long long fluid = 0;
