@@ -185,8 +185,9 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks);
  * serialisation (the next step's blocks are scheduled while the previous step drains).
  * -1 (the default), by grid size from a sweep on GB300: rows narrower than 256 cells: 0; plain
  * FP32: 19 below 2^17 cells, 17 below 2^21, above a ring of its own (4 consumer warps, 2 passes,
- * 2 stages, 5 blocks per SM; reported as 23); 16-bit storage: 19 below 2^21 cells, 20 with rows
- * of at least 2048 cells and 2^22 to 2^25 cells, 17 otherwise; FP64: kernels of
+ * 2 stages, 5 blocks per SM; reported as 23); 16-bit storage: 19 below 2^21 cells, 17 below
+ * 2^22 and on rows that fill 2048-cell tiles badly, else 20 (from 2^23 cells on with 2 blocks per
+ * SM; reported as 27); FP64: kernels of
  * their own that multiply on the integer units, bit for bit the same (25: a ring, 26: the direct
  * kernel, for rows below 256 cells or whose 256-cell tiles are less than 95 % full).
  * With -1 and no launch shape set, runs of at least 4 steps of an FP32 or 16-bit grid that fits the

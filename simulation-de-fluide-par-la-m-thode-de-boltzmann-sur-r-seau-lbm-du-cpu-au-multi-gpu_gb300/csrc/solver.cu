@@ -250,6 +250,10 @@ int launch_ring_t(lbm_solver* s, int steps) {
 // blocks 89.0k / 90.9k / 79k (3000 x 5000: 87.9k / 91.1k / 79k; 2048^2: 85.4k / 87.8k / 84.6k).
 constexpr int kVariantF32Large = 23;
 
+// Internal variant of the automatic choice: 20 with at most 2 resident blocks per SM, for 16-bit
+// storage on grids of at least 2^23 cells.
+constexpr int kVariant16Large = 27;
+
 // Internal variants of the automatic choice in FP64: ring and direct kernel with integer
 // multiplications.
 constexpr int kVariantF64Ring = 25, kVariantF64Direct = 26;
@@ -271,7 +275,9 @@ constexpr int kVariantResident = 24;
 // 143.0k), 4096^2 v20 168.7k (v17 159.3k). With the one-instruction stochastic conversion
 // (fewer instructions per cell) the 16-bit sweep moved on the largest grids (walled channel,
 // seeded state, best of 3): 2048^2 v20 170.6k (v17 149.7k), 4096^2 v20 169.5k (v17 169.0k,
-// v22 170.3k), 8192^2 v17 175.7k (v20 168.9k), so grids of at least 2^25 cells take v17.
+// v22 170.3k), 8192^2 v17 175.7k (v20 168.9k). Variant 20 kept to 2 resident blocks per SM (27)
+// queues less in front of HBM: 4096^2 174.2k, 6144 x 4096 176.2k (v17 171.9k), 8192^2 178.1k; at
+// 2048^2, whose states lie half in L2, 153.8k against 171k with 3 blocks.
 // Rows narrower than 256 cells take the
 // direct kernel (0), whose 128-cell chunks leave fewer lanes idle than the rings' wide tiles
 // (FP64 on 100 x 2000: the ring 12 reached 1.0k MLUPS with a fifth of its lanes busy). FP64
@@ -291,8 +297,8 @@ int auto_variant(const lbm_solver* s) {
   }
   if (sizeof(ST) == 2) {
     if (cells < (2LL << 20)) return 19;
-    if (cells >= (32LL << 20)) return 17;
-    return (s->nx >= 2048 && cells >= (4LL << 20)) ? 20 : 17;  // 2048-cell tiles need wide rows
+    if (cells < (4LL << 20) || !wide_tiles16(s->nx)) return 17;
+    return cells < (8LL << 20) ? 20 : kVariant16Large;
   }
   return cells < (1LL << 17) ? 19 : (cells < (2LL << 20) ? 17 : kVariantF32Large);
 }
@@ -326,6 +332,7 @@ int launch_steps_o(lbm_solver* s, int steps) {
     case 19: return launch_ring_t<ST, kOpen, 8, 1, 4, 3>(s, steps);
     case 20: return launch_ring_t<ST, kOpen, 8, 4, 2, 2>(s, steps);
     case 21: return launch_ring_t<ST, kOpen, 4, 4, 2, 5>(s, steps);
+    case kVariant16Large: return launch_ring_t<ST, kOpen, 8, 4, 2, 2, sizeof(ST) == 2 ? 2 : 0>(s, steps);
     case kVariantF32Large: return launch_ring_t<ST, kOpen, 4, 2, 2, 5, 5>(s, steps);
     case 22: return launch_ring_t<ST, kOpen, 8, 4, 3, 2>(s, steps);
     default: return launch_steps_t<ST, kOpen, 0>(s, steps);

@@ -213,7 +213,7 @@ struct lbm_strips {
   cudaGraphExec_t graph = nullptr;
   int graph_cur = -1;
   bool graphs = true;
-  int passes = 2;  // ring passes per strip: 4 (2048-cell tiles) for 16-bit storage on rows >= 2048
+  int passes = 2;  // ring passes per strip: 4 (2048-cell tiles) for 16-bit storage where they suit
   int sm_count = 0;
   bool direct = false;  // kernels reach host memory
   std::string err;
@@ -290,7 +290,11 @@ int steps_tc(lbm_strips* h, int steps) {
   const auto kernel = strip_ring_kernel<ST, Phys, kOpen, kW, kC, kMin>;
   size_t smem = strip_ring_smem<ST, Phys, kW, kC>() +
                 (h->strips <= kStripTableSmem ? h->strips * sizeof(StripTile) : 0);
-  if (kW == 4) smem = std::max(smem, smem_for_blocks(kMin));  // no more than kMin blocks
+  // No more blocks than HBM needs, as in the solver: 5 narrow ones in FP32, 2 wide ones with 16-bit
+  // storage on large grids.
+  const long long cells = static_cast<long long>(h->nx) * h->ny;
+  if (kW == 4) smem = std::max(smem, smem_for_blocks(kMin));
+  if (kC == 4 && cells >= (8LL << 20)) smem = std::max(smem, smem_for_blocks(2));
   S_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   int per_sm = 0;
   S_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, S::kThreads, smem));
@@ -593,10 +597,9 @@ int lbm_strips_create(int nx, int ny, const uint8_t* solid, double tau, double f
   if (e == cudaSuccess) e = cudaMalloc(&h->views_d, strips * sizeof(StripView));
   if (e == cudaSuccess) e = cudaMemcpy(h->views_d, views.data(), strips * sizeof(StripView), cudaMemcpyHostToDevice);
   // The step kernel's strip table (its tiles: the ring shape of 8 consumer warps x 2 passes, 512
-  // cells per tile, 1024 with 16-bit storage, or 4 passes for 16-bit storage on rows of at
-  // least 2048 cells, over the owned rows, strip after strip).
+  // cells per tile, 1024 with 16-bit storage, or 4 passes for 16-bit storage on wide rows, over the owned rows, strip after strip).
   {
-    h->passes = (elem == 2 && nx >= 2048) ? 4 : 2;
+    h->passes = (elem == 2 && wide_tiles16(nx)) ? 4 : 2;
     std::vector<StripTile> tt(strips);
     for (int k = 0; k < strips; ++k) {
       const int up = k == strips - 1 ? 0 : k + 1, dn = k == 0 ? strips - 1 : k - 1;
