@@ -503,11 +503,10 @@ struct lbm_batch {
   // device: [0] step counter, [1] error flag of the bounded waits, [2] state number of resident
   // launches (never put back)
   uint32_t* step_d = nullptr;
-  // Resident launches: block table, instance cuts and outboxes in one allocation (null: the
-  // ensemble does not fit), used while the caller has chosen no launch shape.
-  char* res_d = nullptr;
+  // Resident launches: block table and instance cuts behind the mask words, outboxes behind buf[1]
+  // (res_blocks 0: the ensemble does not fit); used while the caller has chosen no launch shape.
   int res_blocks = 0, res_force = kForceNone;
-  size_t res_inst_at = 0, res_out_at = 0;
+  size_t res_block_at = 0, res_inst_at = 0, res_out_at = 0;
   bool chosen = false;
   int sm_count = 0, device = 0;
   bool direct = false;  // kernels reach host memory
@@ -887,9 +886,9 @@ int launch_resident_k(lbm_batch* b, int steps) {
   while (steps > 0) {
     const int n = std::min(steps, kResidentSteps);
     B_CUDA(b, cudaLaunchKernelEx(&cfg, kernel, static_cast<const StagedArgs<ST, Phys>*>(b->args_d), b->cur,
-                                 reinterpret_cast<const ResBlock*>(b->res_d),
-                                 reinterpret_cast<const ResInst*>(b->res_d + b->res_inst_at), n,
-                                 reinterpret_cast<LLWord*>(b->res_d + b->res_out_at),
+                                 reinterpret_cast<const ResBlock*>(reinterpret_cast<char*>(b->mask_d) + b->res_block_at),
+                                 reinterpret_cast<const ResInst*>(reinterpret_cast<char*>(b->mask_d) + b->res_inst_at), n,
+                                 reinterpret_cast<LLWord*>(static_cast<char*>(b->buf[1]) + b->res_out_at),
                                  static_cast<const uint32_t*>(b->step_d + 2), reinterpret_cast<int*>(b->step_d + 1)));
     B_CUDA(b, launch_dependent(resident_counter_add, dim3(1), dim3(1), 0, b->stream, b->step_d,
                                static_cast<uint32_t>(n)));
@@ -912,15 +911,16 @@ int launch_resident(lbm_batch* b, int steps) {
 }
 
 // Cuts the ensemble for resident launches: the smallest number of items per tile for which all
-// instances' tiles are at most one per SM. Leaves res_d null where there is none.
+// instances' tiles are at most one per SM. Appends the block table and the cuts to the mask words
+// and returns the outboxes' bytes; 0 where there is no such cut.
 template <int kElem>
-int plan_resident(lbm_batch* b) {
+size_t plan_resident(lbm_batch* b, std::vector<uint32_t>& words) {
   int coop = 0, optin = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, b->device);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
   if (!coop || static_cast<size_t>(optin) < kResSmemBytes + 1024 || b->count > b->sm_count ||
       b->total_cells > static_cast<long long>(b->sm_count) * (kResPlaneBytes / kElem))
-    return LBM_OK;
+    return 0;
   std::vector<ResLayout> cut(b->count), best;
   // The fewest items that fit, by bisection (fewer items, more tiles), from the even share on.
   const long long per_item = kElem == 2 ? 64 : 32;
@@ -939,36 +939,34 @@ int plan_resident(lbm_batch* b) {
       lo = items + 1;
     }
   }
-  if (best.empty()) return LBM_OK;
+  if (best.empty()) return 0;
   std::vector<ResBlock> blocks;
   std::vector<ResInst> insts(b->count);
-  long long words = 0;
+  long long out_words = 0;
   for (int k = 0; k < b->count; ++k) {
-    insts[k] = ResInst{best[k], words};
+    insts[k] = ResInst{best[k], out_words};
     const int tiles = best[k].tx * best[k].ty;
     for (int t = 0; t < tiles; ++t) blocks.push_back(ResBlock{k, t});
-    words += 2LL * best[k].words() * tiles;
+    out_words += 2LL * best[k].words() * tiles;
     const int force = b->inst[k].fy != 0 ? kForceXY : (b->inst[k].fx != 0 ? kForceX : kForceNone);
     b->res_force = std::max(b->res_force, force);
   }
-  auto up = [](size_t n) { return (n + 255) / 256 * 256; };
-  b->res_inst_at = up(blocks.size() * sizeof(ResBlock));
-  b->res_out_at = b->res_inst_at + up(insts.size() * sizeof(ResInst));
-  const size_t out_bytes = static_cast<size_t>(words) * sizeof(LLWord);
-  std::vector<char> tables(b->res_out_at);
-  std::memcpy(tables.data(), blocks.data(), blocks.size() * sizeof(ResBlock));
-  std::memcpy(tables.data() + b->res_inst_at, insts.data(), insts.size() * sizeof(ResInst));
-  B_CUDA(b, cudaMalloc(&b->res_d, b->res_out_at + out_bytes));
-  B_CUDA(b, cudaMemcpy(b->res_d, tables.data(), tables.size(), cudaMemcpyHostToDevice));
-  B_CUDA(b, cudaMemset(b->res_d + b->res_out_at, 0, out_bytes));  // words of no state
+  auto append = [&](const void* data, size_t bytes) {  // at the next 256-byte boundary
+    const size_t at = (words.size() * 4 + 255) / 256 * 256;
+    words.resize((at + bytes + 3) / 4);
+    std::memcpy(reinterpret_cast<char*>(words.data()) + at, data, bytes);
+    return at;
+  };
+  b->res_block_at = append(blocks.data(), blocks.size() * sizeof(ResBlock));
+  b->res_inst_at = append(insts.data(), insts.size() * sizeof(ResInst));
   b->res_blocks = static_cast<int>(blocks.size());
-  return LBM_OK;
+  return static_cast<size_t>(out_words) * sizeof(LLWord);
 }
 
 // Runs `steps` steps: a resident launch where the ensemble fits and the caller has chosen no
 // launch shape, else whole graphs of kGraphSteps launches, then the remainder directly.
 int batch_run(lbm_batch* b, int steps) {
-  if (b->res_d && !b->chosen && steps >= kResidentMinSteps) return launch_resident(b, steps);
+  if (b->res_blocks && !b->chosen && steps >= kResidentMinSteps) return launch_resident(b, steps);
   if (steps >= kGraphSteps && (b->graph == nullptr || b->graph_cur != b->cur)) {
     drop_graph(b);
     if (int rc = batch_dispatch(b, 0, true)) return rc;  // table and grid, outside the capture
@@ -1260,10 +1258,14 @@ int lbm_batch_create(int count, const int* nx, const int* ny, const uint8_t* con
     return fail(LBM_ERR_CUDA);
   b->direct = host_memory_direct(b->device);
   const size_t bytes = static_cast<size_t>(off) * elem + 256;
+  const size_t out_bytes =
+      elem == 4 ? plan_resident<4>(b, all_words) : (elem == 2 ? plan_resident<2>(b, all_words) : 0);
+  b->res_out_at = (bytes + 255) / 256 * 256;  // outboxes: zeros are words of no state
   cudaError_t e = cudaSuccess;
   for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
-    e = cudaMalloc(&b->buf[k], bytes);
-    if (e == cudaSuccess) e = cudaMemset(b->buf[k], 0, bytes);
+    const size_t size = k == 1 && out_bytes ? b->res_out_at + out_bytes : bytes;
+    e = cudaMalloc(&b->buf[k], size);
+    if (e == cudaSuccess) e = cudaMemset(b->buf[k], 0, size);
   }
   if (e == cudaSuccess) e = cudaMalloc(&b->mask_d, all_words.size() * sizeof(uint32_t));
   if (e == cudaSuccess)
@@ -1273,8 +1275,6 @@ int lbm_batch_create(int count, const int* nx, const int* ny, const uint8_t* con
   if (e == cudaSuccess) e = cudaMalloc(&b->step_d, 4 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(b->step_d, 0, 4 * sizeof(uint32_t));
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? LBM_ERR_OUT_OF_MEMORY : LBM_ERR_CUDA);
-  if (elem != 8)
-    if (const int rc = elem == 4 ? plan_resident<4>(b) : plan_resident<2>(b)) return fail(rc);
   *out = b;
   return LBM_OK;
 }
@@ -1284,7 +1284,7 @@ int lbm_batch_destroy(lbm_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   drop_graph(b);
   for (void* p : {b->buf[0], b->buf[1], static_cast<void*>(b->mask_d), b->table_d, b->args_d, b->plans_d, b->ops_d, b->stage,
-                  static_cast<void*>(b->red), static_cast<void*>(b->step_d), static_cast<void*>(b->res_d)})
+                  static_cast<void*>(b->red), static_cast<void*>(b->step_d)})
     cudaFree(p);
   for (cudaEvent_t ev : b->ev)
     if (ev) cudaEventDestroy(ev);
@@ -1426,7 +1426,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
       if (std::getline(ls, k, '\t') && k == key && (ls >> G >> blk >> grd)) {
         ls >> w >> c >> s;
         const Cand cand{G, blk, grd / std::max(1, b->sm_count), w, c, s, 0.0};
-        if ((cand.per_sm != 0 || b->res_d || b->elem == 8) && apply(cand) == LBM_OK) {
+        if ((cand.per_sm != 0 || b->res_blocks || b->elem == 8) && apply(cand) == LBM_OK) {
           b->grid = grd;
           b->tune_report = "cached: " + describe(cand);
           if (report && report_size) std::snprintf(report, report_size, "%s", b->tune_report.c_str());
@@ -1489,7 +1489,7 @@ int lbm_batch_autotune(lbm_batch* b, const char* cache_path, char* report, size_
   if (H == V)
     for (int blk : {128, 256})
       for (int per_sm : {1, 2, 4, 8}) cands.push_back({V, blk, per_sm, 8, 2, 2, 0.0});
-  if (b->res_d || b->elem == 8) cands.push_back({0, kBatchThreads, 0, b->ring_w, b->ring_c, b->ring_s, 0.0});
+  if (b->res_blocks || b->elem == 8) cands.push_back({0, kBatchThreads, 0, b->ring_w, b->ring_c, b->ring_s, 0.0});
   double best = 1e30;
   Cand pick = cands.front();
   std::ostringstream rep;

@@ -634,18 +634,24 @@ int solver_mass_into(lbm_solver* s, const void* state, double* partials, int blo
 
 void pack_mask(const uint8_t* solid, int nx, int ny, int mask_words, std::vector<uint32_t>& out) {
   out.assign(static_cast<size_t>(mask_words) * ny, 0xffffffffu);
+  const int used = (nx + 2 + 31) / 32;  // words that hold cells or periodic neighbours
   for (int y = 0; y < ny; ++y) {
     uint32_t* row = out.data() + static_cast<size_t>(y) * mask_words;
     const uint8_t* src = solid + static_cast<size_t>(y) * nx;
-    auto set = [&](int bit, bool v) {
-      if (v)
-        row[bit >> 5] |= 1u << (bit & 31);
-      else
-        row[bit >> 5] &= ~(1u << (bit & 31));
-    };
-    set(0, src[nx - 1] != 0);
-    for (int x = 0; x < nx; ++x) set(x + 1, src[x] != 0);
-    set(nx + 1, src[0] != 0);
+    for (int q = 0; q < used; ++q) {
+      const int x0 = 32 * q - 1;  // bit 0's cell
+      uint32_t v = 0;
+      if (x0 >= 0 && x0 + 32 <= nx) {
+        for (int j = 0; j < 32; ++j) v |= static_cast<uint32_t>(src[x0 + j] != 0) << j;
+      } else {
+        for (int j = 0; j < 32; ++j) {
+          const int x = x0 + j;
+          const bool s = x < 0 ? src[nx - 1] != 0 : (x < nx ? src[x] != 0 : (x == nx ? src[0] != 0 : true));
+          v |= static_cast<uint32_t>(s) << j;
+        }
+      }
+      row[q] = v;
+    }
   }
 }
 
