@@ -317,13 +317,15 @@ struct BatchFlatPolicy {
     if (lane < 3 * (S::WPS + 1)) mine = sm[(lane / (S::WPS + 1)) * S::MW + sd.w0 + lane % (S::WPS + 1)];
     const bool solids = __any_sync(0xffffffffu, mine != 0u);
     if constexpr (S::LC == 2) {
+      with_force(p.k.force, [&](auto kind) {
 #pragma unroll 1
-      for (int c = 0; c < kC; ++c) {
-        const int x = sd.x0 + 64 * c + 2 * lane;
-        if (x < p.g.nx)
-          ring_pair<ST, false, S, kRows>(p, st, sm, wr, sd.y, x, sd.lx0 + 64 * c + 2 * lane, sd.w0 + 2 * c, lane,
-                                         solids, rkey);
-      }
+        for (int c = 0; c < kC; ++c) {
+          const int x = sd.x0 + 64 * c + 2 * lane;
+          if (x < p.g.nx)
+            ring_pair<ST, decltype(kind)::value, false, S, kRows>(p, st, sm, wr, sd.y, x, sd.lx0 + 64 * c + 2 * lane,
+                                                                  sd.w0 + 2 * c, lane, solids, rkey);
+        }
+      });
     } else {
       with_force(p.k.force, [&](auto kind) {
 #pragma unroll 1
@@ -898,15 +900,18 @@ int launch_resident_k(lbm_batch* b, int steps) {
   return LBM_OK;
 }
 
+template <class ST>
+int launch_resident_f(lbm_batch* b, int steps) {
+  int rc = LBM_OK;
+  with_force(b->res_force, [&](auto kind) { rc = launch_resident_k<ST, decltype(kind)::value>(b, steps); });
+  return rc;
+}
+
 int launch_resident(lbm_batch* b, int steps) {
   switch (b->precision) {
-    case LBM_FP16_STORE: return launch_resident_k<__half, kForceXY>(b, steps);
-    case LBM_BF16_STORE: return launch_resident_k<__nv_bfloat16, kForceXY>(b, steps);
-    default: {
-      int rc = LBM_OK;
-      with_force(b->res_force, [&](auto kind) { rc = launch_resident_k<float, decltype(kind)::value>(b, steps); });
-      return rc;
-    }
+    case LBM_FP16_STORE: return launch_resident_f<__half>(b, steps);
+    case LBM_BF16_STORE: return launch_resident_f<__nv_bfloat16>(b, steps);
+    default: return launch_resident_f<float>(b, steps);
   }
 }
 

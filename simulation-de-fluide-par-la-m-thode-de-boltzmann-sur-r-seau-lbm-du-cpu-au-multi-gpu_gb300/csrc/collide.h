@@ -333,6 +333,7 @@ struct FastConsts {
   float w0, wax, wdg;  // S w_0, S w_axis, S w_diagonal
   float wk3[kQ];       // S w_i 3 fp cf_i
   float wk9[kQ];       // S w_i 9 fp cf_i
+  int force;           // force kind, as CollideConsts::force
 };
 
 inline FastConsts make_fast_consts(float tau, float fx, float fy, float scale = 1.0f) {
@@ -354,6 +355,7 @@ inline FastConsts make_fast_consts(float tau, float fx, float fy, float scale = 
     c.wk3[i] = w * (3.0f * fp * cf);
     c.wk9[i] = w * (9.0f * fp * cf);
   }
+  c.force = fy != 0.0f ? kForceXY : (fx != 0.0f ? kForceX : kForceNone);
   return c;
 }
 
@@ -381,23 +383,28 @@ struct FastF32 {
   }
 };
 
-// Outputs of one pair of opposite directions i (cu) and j (-cu) of weight class (wa, wb, wc).
-template <class P>
-LBM_HD void fast_pair(const typename P::T (&g)[kQ], const FastConsts& kc, int i, int j,
-                      typename P::T cu, typename P::T wa, typename P::T wb, typename P::T wc,
-                      typename P::T om1, typename P::T (&out)[kQ]) {
+// Outputs of one pair of opposite directions i (cu) and j (-cu) of weight class (wa, wb, wc), with
+// the force terms k3 = S w 3 fp cf and k9 = S w 9 fp cf, or (kDriven false) none.
+template <class P, bool kDriven>
+LBM_HD void fast_pair(const typename P::T (&g)[kQ], int i, int j, typename P::T cu, typename P::T wa,
+                      typename P::T wb, typename P::T wc, typename P::T om1, typename P::T k3,
+                      typename P::T k9, typename P::T (&out)[kQ]) {
   using T = typename P::T;
   const T e = P::fma(P::mul(wc, cu), cu, wa);
-  const T o = P::fma(wb, cu, P::k(kc.wk3[i]));
-  const T en = P::fma(P::k(kc.wk9[i]), cu, e);
+  const T o = kDriven ? P::fma(wb, cu, k3) : P::mul(wb, cu);
+  const T en = kDriven ? P::fma(k9, cu, e) : e;
   out[i] = P::fma(om1, g[i], P::add(en, o));
   out[j] = P::fma(om1, g[j], P::sub(en, o));
 }
 
-template <class P>
+// kForce: the force components that may be non-zero; the terms of the others are zeros, and with
+// fy = 0 those of directions 6 and 8 are those of 5 and 7 with the sign turned, so that fewer
+// constants are held and the values are the same.
+template <class P, int kForce = kForceXY>
 LBM_HD void collide_fast_t(const typename P::T (&g)[kQ], const FastConsts& kc,
                            typename P::T (&out)[kQ]) {
   using T = typename P::T;
+  constexpr bool kX = kForce != kForceNone, kY = kForce == kForceXY;
   const T m0s = P::add(P::add(P::add(P::add(g[0], g[1]), P::add(g[2], g[3])),
                               P::add(P::add(g[4], g[5]), P::add(g[6], g[7]))), g[8]);
   const T mxs = P::add(P::add(P::sub(g[1], g[3]), P::sub(g[5], g[6])), P::sub(g[8], g[7]));
@@ -405,21 +412,30 @@ LBM_HD void collide_fast_t(const typename P::T (&g)[kQ], const FastConsts& kc,
   const T m0 = P::mul(m0s, P::k(kc.inv_scale));
   const T rho = P::add(P::k(1.0f), m0);
   const T invs = P::mul(P::rcp(rho), P::k(kc.inv_scale));
-  const T ux = P::mul(P::add(mxs, P::k(kc.shfx)), invs);
-  const T uy = P::mul(P::add(mys, P::k(kc.shfy)), invs);
+  const T ux = P::mul(kX ? P::add(mxs, P::k(kc.shfx)) : mxs, invs);
+  const T uy = P::mul(kY ? P::add(mys, P::k(kc.shfy)) : mys, invs);
   const T usq = P::fma(ux, ux, P::mul(uy, uy));
   const T orho = P::mul(P::k(kc.omega), rho);
-  const T uf = P::fma(P::k(kc.fp3fx), ux, P::mul(P::k(kc.fp3fy), uy));
-  const T a = P::fma(P::k(kc.omega), m0, P::fma(P::mul(P::k(-1.5f), orho), usq, P::neg(uf)));
+  const T m15 = P::mul(P::k(-1.5f), orho);
+  T au;  // -1.5 omega rho |u|^2 - 3 fp (u.F)
+  if (kY)
+    au = P::fma(m15, usq, P::neg(P::fma(P::k(kc.fp3fx), ux, P::mul(P::k(kc.fp3fy), uy))));
+  else if (kX)
+    au = P::fma(m15, usq, P::neg(P::mul(P::k(kc.fp3fx), ux)));
+  else
+    au = P::mul(m15, usq);
+  const T a = P::fma(P::k(kc.omega), m0, au);
   const T b = P::mul(P::k(3.0f), orho), c = P::mul(P::k(4.5f), orho);
   const T om1 = P::k(kc.one_minus_omega);
   out[0] = P::fma(om1, g[0], P::mul(P::k(kc.w0), a));
   const T wa = P::mul(P::k(kc.wax), a), wb = P::mul(P::k(kc.wax), b), wc = P::mul(P::k(kc.wax), c);
-  fast_pair<P>(g, kc, 1, 3, ux, wa, wb, wc, om1, out);
-  fast_pair<P>(g, kc, 2, 4, uy, wa, wb, wc, om1, out);
+  const T k35 = P::k(kc.wk3[5]), k95 = P::k(kc.wk9[5]);
+  fast_pair<P, kX>(g, 1, 3, ux, wa, wb, wc, om1, P::k(kc.wk3[1]), P::k(kc.wk9[1]), out);
+  fast_pair<P, kY>(g, 2, 4, uy, wa, wb, wc, om1, P::k(kc.wk3[2]), P::k(kc.wk9[2]), out);
   const T da = P::mul(P::k(kc.wdg), a), db = P::mul(P::k(kc.wdg), b), dc = P::mul(P::k(kc.wdg), c);
-  fast_pair<P>(g, kc, 5, 7, P::add(ux, uy), da, db, dc, om1, out);
-  fast_pair<P>(g, kc, 6, 8, P::sub(uy, ux), da, db, dc, om1, out);
+  fast_pair<P, kX>(g, 5, 7, P::add(ux, uy), da, db, dc, om1, k35, k95, out);
+  fast_pair<P, kX>(g, 6, 8, P::sub(uy, ux), da, db, dc, om1, kY ? P::k(kc.wk3[6]) : P::neg(k35),
+                   kY ? P::k(kc.wk9[6]) : P::neg(k95), out);
 }
 
 LBM_HD void collide_fast(const float (&g)[kQ], const FastConsts& k, float (&out)[kQ]) {

@@ -381,16 +381,12 @@ int launch_resident_t(lbm_solver* s, int steps) {
 
 template <class ST>
 int launch_resident(lbm_solver* s, int steps) {
-  if constexpr (sizeof(ST) == 4) {
-    int rc = LBM_OK;
-    with_force(Form<ST>::consts(s->tau, s->fx, s->fy).force, [&](auto kind) {
-      constexpr int K = decltype(kind)::value;
-      rc = s->open_x ? launch_resident_t<ST, true, K>(s, steps) : launch_resident_t<ST, false, K>(s, steps);
-    });
-    return rc;
-  } else {
-    return s->open_x ? launch_resident_t<ST, true, kForceXY>(s, steps) : launch_resident_t<ST, false, kForceXY>(s, steps);
-  }
+  int rc = LBM_OK;
+  with_force(Form<ST>::consts(s->tau, s->fx, s->fy).force, [&](auto kind) {
+    constexpr int K = decltype(kind)::value;
+    rc = s->open_x ? launch_resident_t<ST, true, K>(s, steps) : launch_resident_t<ST, false, K>(s, steps);
+  });
+  return rc;
 }
 
 // Do the step kernels' launch sequences end with a counter update?

@@ -200,7 +200,7 @@ __device__ __forceinline__ void res_cell(const StepArgs<ST, Phys>& p, const ST* 
       }
     }
     float2 out[kQ];
-    collide_fast_t<FastF32x2>(v, p.k, out);
+    collide_fast_t<FastF32x2, kForce>(v, p.k, out);
     const uint32_t ph = sr_pair_hash(p.key_base + static_cast<long long>(gy) * p.g.pitch + gx, rkey);
     uint32_t q[kQ];
 #pragma unroll

@@ -180,7 +180,7 @@ __device__ __forceinline__ float2 widen_pair<__nv_bfloat16>(uint32_t raw) {
 // One pair of cells x, x + 1 (x even) of a strip, 16-bit storage, FP32 fast collision. Same
 // stage layout (and kWrapInRow, kHalo) as ring_cell; word / lane locate the pair's mask bits
 // (cells x - 1 .. x + 2); rkey is the step's stochastic-rounding key (step_rkey).
-template <class ST, bool kOpen, class S, bool kWrapInRow = false, bool kHalo = false>
+template <class ST, int kForce, bool kOpen, class S, bool kWrapInRow = false, bool kHalo = false>
 __device__ __forceinline__ void ring_pair(const StepArgs<ST, FastPhys>& p, const ST* st,
                                           const uint32_t* sm, const ST* wr, int y, int x, int lx,
                                           int word, int lane, bool solids, uint32_t rkey) {
@@ -274,7 +274,7 @@ __device__ __forceinline__ void ring_pair(const StepArgs<ST, FastPhys>& p, const
     }
   }
   float2 out[kQ];
-  collide_fast_t<FastF32x2>(v, p.k, out);
+  collide_fast_t<FastF32x2, kForce>(v, p.k, out);
   const uint32_t ph = sr_pair_hash(p.key_base + row + x, rkey);
   uint32_t* d = reinterpret_cast<uint32_t*>(p.dst + row + x);
   uint32_t w[kQ];
@@ -364,13 +364,15 @@ __device__ __forceinline__ void ring_consume_tile(const StepArgs<ST, Phys>& p, c
   if (lane < 3 * (S::WPS + 1)) mine = sm[(lane / (S::WPS + 1)) * S::MW + w0 + lane % (S::WPS + 1)];
   const bool solids = __any_sync(0xffffffffu, mine != 0u);
   if constexpr (S::LC == 2) {
+    with_force(p.k.force, [&](auto kind) {
 #pragma unroll 1
-    for (int c = 0; c < kC; ++c) {
-      const int x = xw + 64 * c + 2 * lane;
-      if (x < nx)
-        ring_pair<ST, kOpen, S, false, kHalo>(p, st, sm, wr, y, x, x - tx0 + S::H, w0 + 2 * c, lane, solids,
-                                              step_rkey(p));
-    }
+      for (int c = 0; c < kC; ++c) {
+        const int x = xw + 64 * c + 2 * lane;
+        if (x < nx)
+          ring_pair<ST, decltype(kind)::value, kOpen, S, false, kHalo>(p, st, sm, wr, y, x, x - tx0 + S::H, w0 + 2 * c,
+                                                                       lane, solids, step_rkey(p));
+      }
+    });
   } else {
     with_force(p.k.force, [&](auto kind) {
 #pragma unroll 1

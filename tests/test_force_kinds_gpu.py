@@ -40,3 +40,23 @@ def test_large_fp32_ring_equals_direct(gpu_lib, nx, ny):
             s.run(5)
             got.append(s.populations())
     assert np.array_equal(*got)
+
+
+@pytest.mark.parametrize("form", ["fp16", "bf16"])
+@pytest.mark.parametrize("force", [(0.0, 0.0), (1e-5, 0.0), (0.0, 1e-5), (1e-5, 2e-6)])
+@pytest.mark.parametrize("nx,ny,open_x", [(259, 33, False), (259, 33, True), (1500, 640, False)])
+def test_force_kinds_16bit(gpu_lib, form, force, nx, ny, open_x):
+    """16-bit storage: the rings and the resident kernel by force kind against the direct kernel,
+    which evaluates every force term; equal numbers (zeros may differ in sign)."""
+    mask = gpu_lib.geometry.add_block(gpu_lib.make_channel(nx, ny), nx, 30, 41, 9, 17)
+    got = []
+    for variant in (0, -1, 12, 17, 19, 20):
+        with gpu_lib.Solver(nx, ny, 0.7, *force, mask, precision=form) as s:
+            if open_x:
+                s.set_inflow_outflow(0.05)
+            s.set_variant(variant)
+            s.init_equilibrium(1.0, 0.05, 0.01)
+            s.run(9)
+            got.append(s.populations())
+    for g in got[1:]:
+        assert np.array_equal(g, got[0])
