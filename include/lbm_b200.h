@@ -183,16 +183,16 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks);
  * tiles), 2 stages, 2 resident blocks; 21 = 4 consumer warps, 4 passes, 2 stages, 5 blocks;
  * 22 = 20 with 3 stages. The ring variants are launched with programmatic stream
  * serialisation (the next step's blocks are scheduled while the previous step drains).
- * -1 (the default), by grid size from a sweep on GB300: rows narrower than 256 cells: 0; plain
- * FP32: 19 below 2^17 cells, 17 below 2^21, above a ring of its own (4 consumer warps, 2 passes,
- * 2 stages, 5 blocks per SM; reported as 23); 16-bit storage: 19 below 2^21 cells, 17 below
- * 2^22 and on rows that fill 2048-cell tiles badly, else 20 (from 2^23 cells on with 2 blocks per
- * SM; reported as 27); FP64: kernels of
- * their own that multiply on the integer units, bit for bit the same (25: a ring, 26: the direct
- * kernel, for rows below 256 cells or whose 256-cell tiles are less than 95 % full).
+ * -1 (the default), by grid size from sweeps on GB300: rows narrower than 256 cells: 0; plain
+ * FP32: 19 below 2^17 cells, 17 below 2^21, then two rings of its own (4 consumer warps, 2 passes;
+ * 2 stages and 5 blocks per SM, reported as 23, from 44 * 2^20 cells on 3 stages and 3 blocks,
+ * 28); 16-bit storage: 19 below 2^21 cells, 17 below 2^22 and on rows that fill 2048-cell tiles
+ * badly, else 20 (from 2^23 cells on with 2 blocks per SM, 27); FP64: kernels of its own that
+ * multiply on the integer units, bit for bit the same (25: a ring, 26: the direct kernel, for rows
+ * below 256 cells or whose 256-cell tiles are less than 95 % full).
  * With -1 and no launch shape set, runs of at least 4 steps of an FP32 or 16-bit grid that fits the
  * SMs' shared memory (up to about 370k cells in FP32, 750k with 16-bit storage, depending on the
- * shape) keep the state there for the whole call, in one cooperative launch (reported as 24).
+ * shape) keep the state there for the whole call, in one cooperative launch (24).
  * The 16-bit forms round stored populations stochastically (see lbm_create); every variant
  * derives the same random bits, so the variants give the same results. */
 int lbm_set_variant(lbm_solver* s, int variant);

@@ -248,7 +248,10 @@ int launch_ring_t(lbm_solver* s, int steps) {
 // stages faster and keeps too many bytes queued: 4096^2 MLUPS by shape and blocks per SM: 12
 // with 4 blocks 78.5k, 3 blocks 87.1k, 2 blocks 86.4k; 15 with 3 blocks 89.7k; this one with 4 / 5 / 6
 // blocks 89.0k / 90.9k / 79k (3000 x 5000: 87.9k / 91.1k / 79k; 2048^2: 85.4k / 87.8k / 84.6k).
-constexpr int kVariantF32Large = 23;
+// The largest grids take 3 stages and 3 blocks (28): 8192^2 91.1k against 87.9k, 8192 x 6000 91.8k /
+// 88.8k, 10000 x 7000 89.1k / 85.2k, 16384 x 4096 91.3k / 88.3k; 6000^2 84.7k / 91.2k, 5000^2 89.7k /
+// 90.6k.
+constexpr int kVariantF32Large = 23, kVariantF32Largest = 28;
 
 // Internal variant of the automatic choice: 20 with at most 2 resident blocks per SM, for 16-bit
 // storage on grids of at least 2^23 cells.
@@ -300,7 +303,8 @@ int auto_variant(const lbm_solver* s) {
     if (cells < (4LL << 20) || !wide_tiles16(s->nx)) return 17;
     return cells < (8LL << 20) ? 20 : kVariant16Large;
   }
-  return cells < (1LL << 17) ? 19 : (cells < (2LL << 20) ? 17 : kVariantF32Large);
+  if (cells < (2LL << 20)) return cells < (1LL << 17) ? 19 : 17;
+  return cells < (44LL << 20) ? kVariantF32Large : kVariantF32Largest;
 }
 
 template <class ST, bool kOpen>
@@ -334,6 +338,7 @@ int launch_steps_o(lbm_solver* s, int steps) {
     case 21: return launch_ring_t<ST, kOpen, 4, 4, 2, 5>(s, steps);
     case kVariant16Large: return launch_ring_t<ST, kOpen, 8, 4, 2, 2, sizeof(ST) == 2 ? 2 : 0>(s, steps);
     case kVariantF32Large: return launch_ring_t<ST, kOpen, 4, 2, 2, 5, 5>(s, steps);
+    case kVariantF32Largest: return launch_ring_t<ST, kOpen, 4, 2, 3, 1, 3>(s, steps);
     case 22: return launch_ring_t<ST, kOpen, 8, 4, 3, 2>(s, steps);
     default: return launch_steps_t<ST, kOpen, 0>(s, steps);
   }

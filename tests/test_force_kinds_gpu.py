@@ -26,7 +26,7 @@ def test_force_kinds(gpu_lib, orc, real, prec, force, variant):
     assert np.array_equal(got, want)
 
 
-@pytest.mark.parametrize("nx,ny", [(2049, 1025), (8191, 257), (4096, 512)])
+@pytest.mark.parametrize("nx,ny", [(2049, 1025), (8191, 257), (4096, 512), (8200, 5650)])
 def test_large_fp32_ring_equals_direct(gpu_lib, nx, ny):
     """At least 2^21 cells: the automatic ring (256-cell tiles, ragged last tile) against the
     direct kernel."""
