@@ -22,10 +22,10 @@
  *     8: (+,-) (src/common/d2q9.hpp:14-25).
  *   - All work of a solver is issued on its stream (lbm_set_stream); functions returning host
  *     data synchronise that stream.
- *   - Host buffers that kernels can address (pinned / registered memory, and on hosts whose page
- *     tables the GPU uses any memory aligned to its values) are read and written by the library's
- *     kernels (state upload, moments, populations, fields); other host buffers are staged through
- *     device memory with copies. Results are the same either way.
+ *   - Host buffers that are aligned to their values and that kernels can address (pinned or
+ *     registered as a whole; on hosts whose page tables the GPU uses ordinary memory too) are read
+ *     and written by the library's kernels (state upload, moments, populations, fields); other host
+ *     buffers are staged through device memory with copies. Results are the same either way.
  */
 #ifndef LBM_B200_H
 #define LBM_B200_H

@@ -1123,7 +1123,7 @@ int set_pop_t(lbm_batch* b, int k, const void* host) {
   const size_t bytes = static_cast<size_t>(in.nx) * in.ny * kQ * sizeof(T);
   if (int rc = ensure_stage(b, bytes)) return rc;
   const void* view = bytes % 16 == 0 ? host_view(host, bytes, 16, b->direct, false) : nullptr;
-  if (view && reinterpret_cast<uintptr_t>(view) % 16 == 0) {
+  if (view) {
     const long long n16 = static_cast<long long>(bytes / 16);
     copy16_kernel<<<static_cast<int>(std::min<long long>((n16 + 255) / 256, 16LL * b->sm_count)), 256, 0, b->stream>>>(
         static_cast<const uint4*>(view), static_cast<uint4*>(b->stage), n16);

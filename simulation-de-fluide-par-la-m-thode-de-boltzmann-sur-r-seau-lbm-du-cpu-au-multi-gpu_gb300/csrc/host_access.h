@@ -75,17 +75,27 @@ inline bool host_pages_present(void* p, size_t bytes, bool make) {
 }
 
 // The address under which kernels may use the host buffer [p, p + bytes) of `elem`-byte values, or
-// null: it is then copied through device memory. direct: host_memory_direct; output: the buffer
-// will be written.
+// null: it is then copied through device memory, which takes any alignment and any registration.
+// Kernels load and store whole values, so the address has to be a multiple of `elem`; pinned or
+// registered memory has to be so from the first byte to the last, at one range of device
+// addresses. direct: host_memory_direct; output: the buffer will be written.
 inline void* host_view(const void* p, size_t bytes, size_t elem, bool direct, bool output) {
-  cudaPointerAttributes a{};
+  if (bytes == 0 || reinterpret_cast<uintptr_t>(p) % elem != 0) return nullptr;
+  cudaPointerAttributes a{}, end{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (a.type == cudaMemoryTypeHost) return a.devicePointer;
-  if (a.type != cudaMemoryTypeUnregistered || !direct || bytes == 0 || reinterpret_cast<uintptr_t>(p) % elem != 0)
-    return nullptr;
+  if (a.type == cudaMemoryTypeHost) {
+    if (cudaPointerGetAttributes(&end, static_cast<const char*>(p) + bytes - 1) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    const uintptr_t first = reinterpret_cast<uintptr_t>(a.devicePointer), last = reinterpret_cast<uintptr_t>(end.devicePointer);
+    const bool whole = end.type == cudaMemoryTypeHost && first != 0 && last == first + (bytes - 1);
+    return whole && first % elem == 0 ? a.devicePointer : nullptr;
+  }
+  if (a.type != cudaMemoryTypeUnregistered || !direct) return nullptr;
   void* q = const_cast<void*>(p);
   return host_pages_present(q, bytes, output) ? q : nullptr;
 }

@@ -1,0 +1,91 @@
+// Host check of csrc/host_access.h with a stand-in for the CUDA runtime's pointer queries: which host
+// buffers kernels are given in place, and which take a copy. No GPU and no CUDA library involved.
+// Exit status 0 when every answer is the expected one.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+
+#include "host_access.h"
+
+namespace {
+// Registered ranges: [lo, lo + bytes) with device address dev.
+struct Range {
+  uintptr_t lo;
+  size_t bytes;
+  uintptr_t dev;
+};
+Range ranges[2];
+int range_count = 0;
+}  // namespace
+
+extern "C" {
+cudaError_t CUDARTAPI cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+  *a = cudaPointerAttributes{};
+  a->type = cudaMemoryTypeUnregistered;
+  const uintptr_t v = reinterpret_cast<uintptr_t>(p);
+  for (int k = 0; k < range_count; ++k)
+    if (v >= ranges[k].lo && v < ranges[k].lo + ranges[k].bytes) {
+      a->type = cudaMemoryTypeHost;
+      a->hostPointer = const_cast<void*>(p);
+      a->devicePointer = reinterpret_cast<void*>(ranges[k].dev + (v - ranges[k].lo));
+    }
+  return cudaSuccess;
+}
+cudaError_t CUDARTAPI cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t CUDARTAPI cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) {
+  *v = 1;
+  return cudaSuccess;
+}
+}
+
+namespace {
+int bad = 0;
+void expect(bool ok, const char* what) {
+  if (ok) return;
+  std::printf("wrong: %s\n", what);
+  ++bad;
+}
+
+void pinned() {
+  using lbm_b200::host_view;
+  alignas(64) static unsigned char buf[4096];
+  const uintptr_t base = reinterpret_cast<uintptr_t>(buf);
+  const uintptr_t dev = uintptr_t(1) << 44;
+  ranges[0] = {base, sizeof buf, dev};
+  range_count = 1;
+  for (bool direct : {false, true})
+    for (bool output : {false, true}) {
+      expect(host_view(buf, 1024, 4, direct, output) == reinterpret_cast<void*>(dev), "pinned: its device address");
+      expect(host_view(buf + 8, 1024, 8, direct, output) == reinterpret_cast<void*>(dev + 8), "pinned at an aligned offset");
+      expect(host_view(buf, sizeof buf, 4, direct, output) == reinterpret_cast<void*>(dev), "pinned: all of it");
+      for (int off : {1, 2, 3, 5})
+        expect(host_view(buf + off, 1024, 4, direct, output) == nullptr, "pinned, not aligned to 4-byte values");
+      expect(host_view(buf + 4, 1024, 8, direct, output) == nullptr, "pinned, not aligned to 8-byte values");
+      expect(host_view(buf + 8, 1024, 16, direct, output) == nullptr, "pinned, not aligned to 16-byte words");
+      expect(host_view(buf, 0, 4, direct, output) == nullptr, "no bytes");
+    }
+  // A device address of another alignment than the host's.
+  ranges[0] = {base, sizeof buf, dev + 2};
+  expect(host_view(buf, 1024, 4, true, true) == nullptr, "device address not aligned");
+  // A registration that ends inside the buffer, and one whose other half lies elsewhere.
+  ranges[0] = {base, 1000, dev};
+  expect(host_view(buf, 1024, 4, true, false) == nullptr, "registered in part");
+  expect(host_view(buf, 1000, 4, true, false) == reinterpret_cast<void*>(dev), "registered to its end");
+  ranges[0] = {base, 512, dev};
+  ranges[1] = {base + 512, 512, dev + (1 << 20)};
+  range_count = 2;
+  expect(host_view(buf, 1024, 4, true, false) == nullptr, "two registrations, apart on the device");
+  ranges[1].dev = dev + 512;
+  expect(host_view(buf, 1024, 4, true, false) == reinterpret_cast<void*>(dev), "two registrations, one range");
+  range_count = 0;
+}
+}  // namespace
+
+int main(int argc, char** argv) {
+  const std::string which = argc > 1 ? argv[1] : "";
+  if (which == "pinned") pinned();
+  else return 2;
+  std::printf("%s: %d wrong\n", which.c_str(), bad);
+  return bad == 0 ? 0 : 1;
+}
