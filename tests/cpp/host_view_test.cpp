@@ -80,11 +80,60 @@ void pinned() {
   expect(host_view(buf, 1024, 4, true, false) == reinterpret_cast<void*>(dev), "two registrations, one range");
   range_count = 0;
 }
+
+// Pageable memory that cannot be read or written: a copy reports that as an ordinary error of the
+// host, so kernels do not get it.
+void protection() {
+  using lbm_b200::host_view;
+  const size_t page = static_cast<size_t>(sysconf(_SC_PAGESIZE)), pages = 8, bytes = pages * page;
+  auto map = [&](int fd = -1) {
+    void* p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, fd < 0 ? MAP_PRIVATE | MAP_ANONYMOUS : MAP_SHARED, fd, 0);
+    if (p == MAP_FAILED) std::exit(3);
+    return static_cast<unsigned char*>(p);
+  };
+  unsigned char* p = map();
+  expect(host_view(p, bytes, 4, true, true) == p, "fresh output: its pages are made");
+  std::memset(p, 1, bytes);
+  expect(host_view(p, bytes, 4, true, true) == p && host_view(p, bytes, 4, true, false) == p, "present pages");
+  expect(host_view(p, bytes, 4, false, true) == nullptr, "pageable memory out of the device's reach");
+  mprotect(p + 3 * page, page, PROT_READ);
+  expect(host_view(p, bytes, 4, true, true) == nullptr, "output with a read-only page");
+  expect(host_view(p, bytes, 4, true, false) == p, "input with a read-only page");
+  expect(host_view(p, 3 * page, 4, true, true) == p, "output up to the read-only page");
+  mprotect(p + 3 * page, page, PROT_NONE);
+  expect(host_view(p, bytes, 4, true, false) == nullptr, "input with an inaccessible page");
+  expect(host_view(p, bytes, 4, true, true) == nullptr, "output with an inaccessible page");
+  for (size_t k = 0; k < bytes; k += page)
+    if (k != 3 * page) expect(p[k] == 1, "contents kept");
+  munmap(p, bytes);
+  // A read-only mapping from the start, never touched.
+  p = map();
+  mprotect(p, bytes, PROT_READ);
+  expect(host_view(p, bytes, 4, true, true) == nullptr, "fresh read-only output");
+  munmap(p, bytes);
+  // A hole.
+  p = map();
+  std::memset(p, 1, bytes);
+  munmap(p + 2 * page, page);
+  expect(host_view(p, bytes, 4, true, true) == nullptr && host_view(p, bytes, 4, true, false) == nullptr, "unmapped page");
+  munmap(p, bytes);
+  // A shared file that ends inside the mapping.
+  std::FILE* f = std::tmpfile();
+  if (!f || ftruncate(fileno(f), static_cast<off_t>(2 * page))) std::exit(3);
+  p = map(fileno(f));
+  std::memset(p, 1, 2 * page);
+  expect(host_view(p, 2 * page, 4, true, true) == p, "file mapping up to its end");
+  expect(host_view(p, bytes, 4, true, true) == nullptr, "output past the file's end");
+  expect(host_view(p, bytes, 4, true, false) == nullptr, "input past the file's end");
+  munmap(p, bytes);
+  std::fclose(f);
+}
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "pinned") pinned();
+  else if (which == "protection") protection();
   else return 2;
   std::printf("%s: %d wrong\n", which.c_str(), bad);
   return bad == 0 ? 0 : 1;
