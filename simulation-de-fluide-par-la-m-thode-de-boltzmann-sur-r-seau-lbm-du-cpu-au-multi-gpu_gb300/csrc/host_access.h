@@ -18,8 +18,8 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <exception>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -59,7 +59,7 @@ inline bool host_pages_ready(void* p, size_t bytes, bool write) {
     int started = 1;
     try {
       for (; started < n; ++started) more.emplace_back(part, started);
-    } catch (const std::system_error&) {  // no thread to be had: this one does the rest
+    } catch (const std::exception&) {  // no thread, or no memory for one: this one does the rest
     }
     part(0);
     for (int k = started; k < n; ++k) part(k);

@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
 
 #include "host_access.h"
@@ -17,7 +18,18 @@ struct Range {
 };
 Range ranges[2];
 int range_count = 0;
+// Allocations left before operator new fails (negative: no limit).
+long allocations = -1;
 }  // namespace
+
+void* operator new(size_t n) {
+  if (allocations == 0) throw std::bad_alloc();
+  if (allocations > 0) --allocations;
+  if (void* p = std::malloc(n ? n : 1)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 extern "C" {
 cudaError_t CUDARTAPI cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
@@ -128,12 +140,37 @@ void protection() {
   munmap(p, bytes);
   std::fclose(f);
 }
+
+// Memory that runs out at any of the allocations of a large buffer's preparation, also between the
+// starts of its threads: an answer, no exception and no abort.
+void allocation() {
+  const size_t bytes = 32u << 20;
+  int usable = 0;
+  for (long limit = 0; limit < 12; ++limit) {
+    void* p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (p == MAP_FAILED) std::exit(3);
+    allocations = limit;
+    void* v = nullptr;
+    bool thrown = false;
+    try {
+      v = lbm_b200::host_view(p, bytes, 4, true, true);
+    } catch (...) {
+      thrown = true;
+    }
+    allocations = -1;
+    expect(!thrown && (v == nullptr || v == p), "an answer without memory");
+    usable += v == p;
+    munmap(p, bytes);
+  }
+  expect(usable > 0 && usable < 12, "limits on both sides of what a preparation takes");
+}
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "pinned") pinned();
   else if (which == "protection") protection();
+  else if (which == "allocation") allocation();
   else return 2;
   std::printf("%s: %d wrong\n", which.c_str(), bad);
   return bad == 0 ? 0 : 1;

@@ -23,7 +23,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("part", ["pinned", "protection"])
+@pytest.mark.parametrize("part", ["pinned", "protection", "allocation"])
 def test_host_view(exe, part):
     r = subprocess.run([str(exe), part], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
