@@ -331,7 +331,7 @@ __device__ __forceinline__ typename A::T collide_cell_drag(const typename A::T (
                                                            typename A::T alpha, typename A::T (&out)[kQ]) {
   typename A::T ux = collide_exact_drag<A>(g, k, alpha, out);
   if constexpr (std::is_same_v<A, ExactF64Int>) {
-    if (any_nan(out)) {
+    if (any_nan(out, ux)) {
       double v[kQ], o[kQ];
 #pragma unroll
       for (int i = 0; i < kQ; ++i) v[i] = g[i];

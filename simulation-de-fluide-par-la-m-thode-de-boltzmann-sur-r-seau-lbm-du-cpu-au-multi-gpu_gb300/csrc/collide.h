@@ -220,8 +220,9 @@ LBM_HD void collide_exact_post(const typename A::T (&g)[kQ], typename A::T omega
   }
 }
 
+// Returns u_x.
 template <class A, int kForce>
-LBM_HD void collide_exact_kind(const typename A::T (&g)[kQ], const CollideConsts<typename A::T>& k,
+LBM_HD typename A::T collide_exact_kind(const typename A::T (&g)[kQ], const CollideConsts<typename A::T>& k,
                                typename A::T (&out)[kQ]) {
   using T = typename A::T;
   using S = typename A::S;
@@ -233,6 +234,7 @@ LBM_HD void collide_exact_kind(const typename A::T (&g)[kQ], const CollideConsts
   const T uy = A::div(kForce == kForceXY ? A::add(my, k.hfy) : my, rho);
   collide_exact_post<A, kForce>(g, k.omega, k.force_prefactor, drho, rho, ux, uy, k.cf_x, k.cf_y, k.cf_p,
                                 k.cf_q, out);
+  return ux;
 }
 
 // Calls f(ForceKind<kind>) for a run-time force kind. The kind is the same for

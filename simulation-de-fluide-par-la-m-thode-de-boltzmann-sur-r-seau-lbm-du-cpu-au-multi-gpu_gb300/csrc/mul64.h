@@ -8,10 +8,12 @@
 // The method is the schoolbook one of IEEE 754 arithmetic: the 53-bit significands are multiplied
 // exactly (four 32 x 32 -> 64 products; the second factor is held 11 bits up, so that the high 64
 // bits of the 117-bit product hold 52 or 53 significant ones), normalised by one bit, and rounded
-// to nearest even from the bits below. Factors that are zero give zero (of positive sign: the
-// exact forms treat -0 as +0). Factors outside [2^-400, 2^400), infinities and NaNs give NaN:
-// the collision checks its results for NaN and takes the hardware's multiplications then
-// (collide_cell).
+// to nearest even from the bits below. A factor of zero gives zero (of positive sign: the exact
+// forms treat -0 as +0), also with an infinite or NaN one, which IEEE 754 makes NaN; other factors
+// outside [2^-400, 2^400), infinities and NaNs give NaN. The collision checks its results and its
+// velocity and takes the hardware's multiplications where one of them is not finite
+// (collide_cell; telling 0 * inf apart in every product costs 2 % on the ring and 14 % on the
+// direct kernel, 300 x 300 3270 -> 2800 MLUPS).
 #pragma once
 
 #include <cstdint>

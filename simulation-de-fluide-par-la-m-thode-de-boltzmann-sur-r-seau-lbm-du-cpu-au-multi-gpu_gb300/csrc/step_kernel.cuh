@@ -55,9 +55,14 @@ __device__ __forceinline__ uint32_t step_rkey(const StepArgs<ST, Phys>& p) {
   return sr_step_key(__ldg(p.step_ctr) + p.step_off);
 }
 
-// Is any of the values NaN (or infinite)?
-__device__ __forceinline__ bool any_nan(const double (&v)[kQ]) {
-  uint32_t top = 0;
+// Did integer multiplications (ExactF64Int) give a cell that the hardware's may not: is one of its
+// results, or its velocity ux, NaN or infinite? The results alone would not tell: an integer product
+// of zero and a non-finite factor is zero. What is not finite reaches direction 0's result through
+// w_0 (drho - rho 1.5 |u|^2), and so does a factor outside the integer form's range, unless the
+// density rho is zero; then u = m / rho is not finite (with a drag too: its divisor is a multiple
+// of rho).
+__device__ __forceinline__ bool any_nan(const double (&v)[kQ], double ux) {
+  uint32_t top = static_cast<uint32_t>(__double2hiint(ux)) & 0x7fffffffu;
 #pragma unroll
   for (int i = 0; i < kQ; ++i) top = max(top, static_cast<uint32_t>(__double2hiint(v[i])) & 0x7fffffffu);
   return top >= 0x7ff00000u;
@@ -72,14 +77,14 @@ __device__ __noinline__ void collide_exact_rare(const typename A::T (&g)[kQ], Co
 }
 
 // The collision of one cell as the step kernels take it. Integer multiplications (ExactF64Int)
-// give NaN for factors outside their range; such a cell, or one that holds a NaN, is collided
-// again with the hardware's.
+// give NaN for factors outside their range; such a cell, or one whose values are not finite, is
+// collided again with the hardware's.
 template <class A, int kForce>
 __device__ __forceinline__ void collide_cell(const typename A::T (&g)[kQ], const CollideConsts<typename A::T>& k,
                                              typename A::T (&out)[kQ]) {
-  collide_exact_kind<A, kForce>(g, k, out);
+  const typename A::T ux = collide_exact_kind<A, kForce>(g, k, out);
   if constexpr (std::is_same_v<A, ExactF64Int>) {
-    if (any_nan(out)) {
+    if (any_nan(out, ux)) {
       double v[kQ], o[kQ];
 #pragma unroll
       for (int i = 0; i < kQ; ++i) v[i] = g[i];
