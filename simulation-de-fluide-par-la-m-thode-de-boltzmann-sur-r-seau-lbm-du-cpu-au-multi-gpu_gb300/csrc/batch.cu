@@ -953,8 +953,8 @@ size_t plan_resident(lbm_batch* b, std::vector<uint32_t>& words) {
     const int tiles = best[k].tx * best[k].ty;
     for (int t = 0; t < tiles; ++t) blocks.push_back(ResBlock{k, t});
     out_words += 2LL * best[k].words() * tiles;
-    const int force = b->inst[k].fy != 0 ? kForceXY : (b->inst[k].fx != 0 ? kForceX : kForceNone);
-    b->res_force = std::max(b->res_force, force);
+    using F = BForm<std::conditional_t<kElem == 2, __half, float>>;
+    b->res_force = std::max(b->res_force, F::consts(b->inst[k].tau, b->inst[k].fx, b->inst[k].fy).force);
   }
   auto append = [&](const void* data, size_t bytes) {  // at the next 256-byte boundary
     const size_t at = (words.size() * 4 + 255) / 256 * 256;

@@ -52,6 +52,17 @@ struct CollideConsts {
 // the Guo source then has fewer distinct terms (collide_exact_kind).
 constexpr int kForceNone = 0, kForceX = 1, kForceXY = 2;
 
+// The force kind of (fx, fy). A force along x below 2^-30 (double: 2^-400) takes the general form:
+// the short one has 4 RN(a / 9) for RN(4 a / 9), which differs where a / 9 is subnormal. From 2^-30
+// on it cannot be: u_x rho = m_x + fx / 2 is zero or at least an ulp of its terms, 2^-55, so that
+// the products u_x fx, (...) 3 / 9 and (...) (1 - omega / 2) stay above 2^-85, 2^-87 and 2^-111
+// (times 1 / rho; double: 2^-855, 2^-857, 2^-910 against 2^-1022).
+template <class T>
+LBM_HD constexpr int force_kind(T fx, T fy) {
+  const T least = sizeof(T) == 8 ? T(0x1p-400) : T(0x1p-30f);
+  return fy != T(0) ? kForceXY : (fx == T(0) ? kForceNone : (fx >= least || -fx >= least ? kForceX : kForceXY));
+}
+
 template <class T>
 inline CollideConsts<T> make_collide_consts(T tau, T fx, T fy) {
   CollideConsts<T> c;
@@ -65,7 +76,7 @@ inline CollideConsts<T> make_collide_consts(T tau, T fx, T fy) {
   c.cf_y = fy;
   c.cf_p = fx + fy;
   c.cf_q = fy - fx;
-  c.force = fy != T(0) ? kForceXY : (fx != T(0) ? kForceX : kForceNone);
+  c.force = force_kind(fx, fy);
   return c;
 }
 
@@ -84,8 +95,9 @@ inline CollideConsts<T> make_collide_consts(T tau, T fx, T fy) {
 //   * products by powers of two are exact, so RN(4.5 a) = RN(9 a) / 2 and RN(RN(4.5 a) a) =
 //     RN(RN(9 a) a) / 2: the 9 a of the Guo source serves the equilibrium too, and the halving
 //     is folded into the following sum by an fma (a single rounding of an exact product plus the
-//     addend: the same sum). Likewise RN(4/9) = 4 RN(1/9) and RN(1/36) = RN(1/9) / 4. Where a
-//     underflows so far that a halving is inexact, the term is below half an ulp of 3 a;
+//     addend: the same sum). Where a is so small that a halving is inexact, the term is far below
+//     half an ulp of 3 a. Likewise RN(4/9) = 4 RN(1/9) and RN(1/36) = RN(1/9) / 4, which the source
+//     along x uses where its products cannot be subnormal (force_kind);
 //   * a force component that is zero contributes zeros (collide_exact_kind).
 // Only the sign of an exact zero can differ from v0 (numerically equal: the reference's tests
 // compare with `!=`). A state holding inf or NaN has diverged; results then differ from v0 only
