@@ -17,7 +17,8 @@ __device__ __forceinline__ long long cell_index(const Grid2D& g, int x, int y) {
 // Post-streaming populations of fluid cell (x, y) from the pull state R: population i arrives
 // from (x - cx_i, y - cy_i) (periodic), or bounces back as R[opp i] of the cell itself when that
 // source is solid; open domain: inlet equilibrium at x = 0 for c_x = +1, outlet copy of column
-// nx - 2 at x = nx - 1 for c_x = -1 (reference src/common/boundary.hpp:53-70).
+// nx - 2 at x = nx - 1 for c_x = -1 (reference src/common/boundary.hpp:53-70), where a solid cell
+// (nx - 2, y) sends nothing back: the step kernels store what they like in solid slots.
 template <class ST>
 __device__ void gather_cell(const ST* __restrict__ R, const uint32_t* __restrict__ mask,
                             const Grid2D& g, int x, int y,
@@ -35,10 +36,12 @@ __device__ void gather_cell(const ST* __restrict__ R, const uint32_t* __restrict
     xs = xs < 0 ? g.nx - 1 : (xs >= g.nx ? 0 : xs);
     int ys = y - dir_cy(i);
     ys = ys < 0 ? g.ny - 1 : (ys >= g.ny ? 0 : ys);
-    if (mask_solid(mask, g.mask_words, xs, ys))
-      out[i] = load_one<ST>(R + dir_opp(i) * g.plane + cell_index(g, xc, y), dir_opp(i), sc);
-    else
+    if (!mask_solid(mask, g.mask_words, xs, ys))
       out[i] = load_one<ST>(R + i * g.plane + cell_index(g, xs, ys), i, sc);
+    else if (xc != x && mask_solid(mask, g.mask_words, xc, y))
+      out[i] = typename StoreTraits<ST>::T(0);
+    else
+      out[i] = load_one<ST>(R + dir_opp(i) * g.plane + cell_index(g, xc, y), dir_opp(i), sc);
   }
 }
 

@@ -306,7 +306,8 @@ __device__ __forceinline__ void process_chunk(const StepArgs<ST, Phys>& p, const
       v[8][0] = p.eq_in[8];
     }
     // Outlet (x = nx - 1): populations entering with c_x = -1 are those the cell x = nx - 2
-    // receives (reference src/v3_cuda_opt/solver_v3.cu:66-73).
+    // receives (reference src/v3_cuda_opt/solver_v3.cu:66-73); where that cell is solid, nothing
+    // bounces back from it.
     const int kl = nx - 1 - x0;
     if (kl >= 0 && kl < G) {
 #pragma unroll
@@ -315,11 +316,11 @@ __device__ __forceinline__ void process_chunk(const StepArgs<ST, Phys>& p, const
         const int r = src_row(i, y, c.ym, c.yp);
         const uint32_t w = dir_cy(i) == 1 ? wm : (dir_cy(i) == -1 ? wp : w0);
         const bool solid_src = (w >> (kl + 1)) & 1u;
-        const T val = solid_src
-                          ? load_step<ST>(p.src + dir_opp(i) * plane +
-                                             static_cast<long long>(y) * pitch + (nx - 2))
-                          : load_step<ST>(p.src + i * plane + static_cast<long long>(r) * pitch +
-                                             (nx - 1));
+        T val = T(0);
+        if (!solid_src)
+          val = load_step<ST>(p.src + i * plane + static_cast<long long>(r) * pitch + (nx - 1));
+        else if (!((w0 >> kl) & 1u))
+          val = load_step<ST>(p.src + dir_opp(i) * plane + static_cast<long long>(y) * pitch + (nx - 2));
 #pragma unroll
         for (int k = 0; k < G; ++k)
           if (k == kl) v[i][k] = val;
@@ -329,8 +330,9 @@ __device__ __forceinline__ void process_chunk(const StepArgs<ST, Phys>& p, const
 
   // Collide each cell and store the 9 planes of the own cells. Solid and padding cells are
   // collided too and their slots receive whatever that gives: no kernel ever reads a solid slot
-  // (a fluid cell whose source is solid bounces back instead, and every gather, moment and
-  // reduction skips solid cells), so no per-cell select is spent on them.
+  // (a fluid cell whose source is solid bounces back instead, an outlet cell beside a solid one takes
+  // zeros, and every gather, moment and reduction skips solid cells), so no per-cell select is
+  // spent on them.
   T out[kQ][G];
   Phys::template collide_all<G>(v, p.k, out);
   if (c.active) {

@@ -140,7 +140,10 @@ __device__ __forceinline__ void res_cell(const StepArgs<ST, Phys>& p, const ST* 
         for (int i = 1; i < kQ; ++i) {
           if (dir_cx(i) != -1) continue;
           const uint32_t b = dir_cy(i) == 1 ? nm : (dir_cy(i) == -1 ? np : n0);
-          v[i] = ((b >> 1) & 1u) ? c[dir_opp(i) * PS - 1] : c[i * PS - dir_cy(i) * rs];
+          if (!((b >> 1) & 1u))
+            v[i] = c[i * PS - dir_cy(i) * rs];
+          else  // nothing from a solid cell nx - 2
+            v[i] = (n0 & 1u) ? 0.0f : c[dir_opp(i) * PS - 1];
         }
       }
     }
@@ -193,8 +196,11 @@ __device__ __forceinline__ void res_cell(const StepArgs<ST, Phys>& p, const ST* 
         for (int i = 1; i < kQ; ++i) {
           if (dir_cx(i) != -1) continue;
           const uint32_t b = dir_cy(i) == 1 ? nm : (dir_cy(i) == -1 ? np : n0);
-          const float t = ((b >> (1 + k)) & 1u) ? widen<ST>(c[dir_opp(i) * PS + k - 1])
-                                                : widen<ST>(c[i * PS - dir_cy(i) * rs + k]);
+          float t = 0.0f;
+          if (!((b >> (1 + k)) & 1u))
+            t = widen<ST>(c[i * PS - dir_cy(i) * rs + k]);
+          else if (!((n0 >> k) & 1u))
+            t = widen<ST>(c[dir_opp(i) * PS + k - 1]);
           if (k == 0) v[i].x = t; else v[i].y = t;
         }
       }

@@ -127,11 +127,12 @@ __device__ __forceinline__ void ring_cell(const StepArgs<ST, ExactPhys<A>>& p, c
       for (int i = 1; i < kQ; ++i) {
         if (dir_cx(i) != -1) continue;
         // Zero-gradient outflow: the source is cell nx - 1 of row y - c_y; bounce-back from cell
-        // nx - 2 of row y when that source is solid.
+        // nx - 2 of row y when that source is solid (nothing from a solid cell nx - 2).
         const uint32_t w = dir_cy(i) == 1 ? nm : (dir_cy(i) == -1 ? np : n0);
-        v[i] = ((w >> 1) & 1u)
-                   ? __ldg(p.src + dir_opp(i) * plane + static_cast<long long>(y) * p.g.pitch + (nx - 2))
-                   : st[i * S::SROW + lx];
+        if (!((w >> 1) & 1u))
+          v[i] = st[i * S::SROW + lx];
+        else
+          v[i] = (n0 & 1u) ? T(0) : __ldg(p.src + dir_opp(i) * plane + static_cast<long long>(y) * p.g.pitch + (nx - 2));
       }
     }
   }
@@ -266,9 +267,11 @@ __device__ __forceinline__ void ring_pair(const StepArgs<ST, FastPhys>& p, const
       for (int i = 1; i < kQ; ++i) {
         if (dir_cx(i) != -1) continue;
         const uint32_t w = dir_cy(i) == 1 ? nm : (dir_cy(i) == -1 ? np : n0);
-        const float val = ((w >> (1 + k)) & 1u)
-                              ? load_step<ST>(p.src + dir_opp(i) * plane + row + (nx - 2))
-                              : widen<ST>(st[i * S::SROW + lx + k]);
+        float val = 0.0f;
+        if (!((w >> (1 + k)) & 1u))
+          val = widen<ST>(st[i * S::SROW + lx + k]);
+        else if (!((n0 >> k) & 1u))
+          val = load_step<ST>(p.src + dir_opp(i) * plane + row + (nx - 2));
         if (k == 0) v[i].x = val; else v[i].y = val;
       }
     }

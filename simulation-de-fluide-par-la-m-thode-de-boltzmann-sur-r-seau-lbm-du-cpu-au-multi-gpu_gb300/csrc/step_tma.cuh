@@ -289,9 +289,11 @@ __device__ __forceinline__ void consume_cells(const StepArgs<ST, Phys>& p, const
         const int r = src_row(i, y, ym, yp);
         const uint32_t w = dir_cy(i) == 1 ? wm : (dir_cy(i) == -1 ? wp : w0);
         const bool solid_src = (w >> (kl + 1)) & 1u;
-        const T val = solid_src
-                          ? load_step<ST>(p.src + dir_opp(i) * plane + static_cast<long long>(y) * pitch + (nx - 2))
-                          : load_step<ST>(p.src + i * plane + static_cast<long long>(r) * pitch + (nx - 1));
+        T val = T(0);
+        if (!solid_src)
+          val = load_step<ST>(p.src + i * plane + static_cast<long long>(r) * pitch + (nx - 1));
+        else if (!((w0 >> kl) & 1u))
+          val = load_step<ST>(p.src + dir_opp(i) * plane + static_cast<long long>(y) * pitch + (nx - 2));
 #pragma unroll
         for (int k = 0; k < G; ++k)
           if (k == kl) v[i][k] = val;
