@@ -42,12 +42,15 @@ inline bool host_pages_ready(void* p, size_t bytes, bool write) {
     const uintptr_t page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
     const uintptr_t lo = reinterpret_cast<uintptr_t>(p) / page * page;
     const uintptr_t hi = (reinterpret_cast<uintptr_t>(p) + bytes + page - 1) / page * page;
-    std::vector<unsigned char> in((hi - lo) / page);
-    if (mincore(reinterpret_cast<void*>(lo), hi - lo, in.data()) != 0) return false;
-    const size_t missing = static_cast<size_t>(std::count_if(in.begin(), in.end(), [](unsigned char c) { return !(c & 1); }));
     // A thread costs about 20 us to start, a page about 10 us to make (48 fresh buffers of 0.1 to
     // 19 MB: 9.8 ms with a thread for each 2 MB, 11.9 ms for each 8 MB) and 0.02 us to look at.
-    const int n = static_cast<int>(std::min<size_t>(4, 1 + missing * page / (2u << 20) + (hi - lo) / (256u << 20)));
+    int n = 1;
+    if (hi - lo > (2u << 20)) {
+      std::vector<unsigned char> in((hi - lo) / page);
+      if (mincore(reinterpret_cast<void*>(lo), hi - lo, in.data()) != 0) return false;
+      const size_t missing = static_cast<size_t>(std::count_if(in.begin(), in.end(), [](unsigned char c) { return !(c & 1); }));
+      n = static_cast<int>(std::min<size_t>(4, 1 + missing * page / (2u << 20) + (hi - lo) / (256u << 20)));
+    }
     const uintptr_t share = ((hi - lo) / page + n - 1) / n * page;
     bool ok[4] = {true, true, true, true};
     auto part = [&](int k) {
