@@ -192,7 +192,8 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks);
  * below 256 cells or whose 256-cell tiles are less than 95 % full).
  * With -1 and no launch shape set, runs of at least 4 steps of an FP32 or 16-bit grid that fits the
  * SMs' shared memory (up to about 370k cells in FP32, 750k with 16-bit storage, depending on the
- * shape) keep the state there for the whole call, in one cooperative launch (24).
+ * shape) keep the state there for the whole call, in one cooperative launch (24); on a stream whose
+ * SMs are fewer than its blocks (a green context) the step kernels take them.
  * The 16-bit forms round stored populations stochastically (see lbm_create); every variant
  * derives the same random bits, so the variants give the same results. */
 int lbm_set_variant(lbm_solver* s, int variant);

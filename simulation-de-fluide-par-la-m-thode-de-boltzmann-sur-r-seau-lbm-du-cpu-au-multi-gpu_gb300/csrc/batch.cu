@@ -35,6 +35,7 @@
 #include "step_kernel.cuh"
 #include "step_resident.cuh"
 #include "step_ring.cuh"
+#include "stream_sms.h"
 
 using namespace lbm_b200;
 
@@ -863,6 +864,9 @@ int batch_steps(lbm_batch* b, int steps) {
   return batch_dispatch(b, steps, false);
 }
 
+// A resident launch that was refused because its blocks cannot all be resident: nothing of it ran.
+constexpr int kRefused = -1;
+
 template <class ST, int kForce>
 int launch_resident_k(lbm_batch* b, int steps) {
   using Phys = typename BForm<ST>::Phys;
@@ -885,17 +889,23 @@ int launch_resident_k(lbm_batch* b, int steps) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  while (steps > 0) {
-    const int n = std::min(steps, kResidentSteps);
-    B_CUDA(b, cudaLaunchKernelEx(&cfg, kernel, static_cast<const StagedArgs<ST, Phys>*>(b->args_d), b->cur,
-                                 reinterpret_cast<const ResBlock*>(reinterpret_cast<char*>(b->mask_d) + b->res_block_at),
-                                 reinterpret_cast<const ResInst*>(reinterpret_cast<char*>(b->mask_d) + b->res_inst_at), n,
-                                 reinterpret_cast<LLWord*>(static_cast<char*>(b->buf[1]) + b->res_out_at),
-                                 static_cast<const uint32_t*>(b->step_d + 2), reinterpret_cast<int*>(b->step_d + 1)));
+  for (int done = 0; done < steps;) {
+    const int n = std::min(steps - done, kResidentSteps);
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, kernel, static_cast<const StagedArgs<ST, Phys>*>(b->args_d), b->cur,
+                           reinterpret_cast<const ResBlock*>(reinterpret_cast<char*>(b->mask_d) + b->res_block_at),
+                           reinterpret_cast<const ResInst*>(reinterpret_cast<char*>(b->mask_d) + b->res_inst_at), n,
+                           reinterpret_cast<LLWord*>(static_cast<char*>(b->buf[1]) + b->res_out_at),
+                           static_cast<const uint32_t*>(b->step_d + 2), reinterpret_cast<int*>(b->step_d + 1));
+    if (e == cudaErrorCooperativeLaunchTooLarge && done == 0) {
+      cudaGetLastError();
+      return kRefused;
+    }
+    B_CUDA(b, e);
     B_CUDA(b, launch_dependent(resident_counter_add, dim3(1), dim3(1), 0, b->stream, b->step_d,
                                static_cast<uint32_t>(n)));
     b->t += static_cast<uint32_t>(n);
-    steps -= n;
+    done += n;
   }
   return LBM_OK;
 }
@@ -968,10 +978,15 @@ size_t plan_resident(lbm_batch* b, std::vector<uint32_t>& words) {
   return static_cast<size_t>(out_words) * sizeof(LLWord);
 }
 
-// Runs `steps` steps: a resident launch where the ensemble fits and the caller has chosen no
-// launch shape, else whole graphs of kGraphSteps launches, then the remainder directly.
+// Runs `steps` steps: a resident launch where the ensemble fits, its blocks the SMs that the stream
+// may use, and the caller has chosen no launch shape, else whole graphs of kGraphSteps launches,
+// then the remainder directly.
 int batch_run(lbm_batch* b, int steps) {
-  if (b->res_blocks && !b->chosen && steps >= kResidentMinSteps) return launch_resident(b, steps);
+  if (b->res_blocks && !b->chosen && steps >= kResidentMinSteps &&
+      b->res_blocks <= stream_sm_count(b->stream, b->sm_count)) {
+    const int rc = launch_resident(b, steps);
+    if (rc != kRefused) return rc;
+  }
   if (steps >= kGraphSteps && (b->graph == nullptr || b->graph_cur != b->cur)) {
     drop_graph(b);
     if (int rc = batch_dispatch(b, 0, true)) return rc;  // table and grid, outside the capture

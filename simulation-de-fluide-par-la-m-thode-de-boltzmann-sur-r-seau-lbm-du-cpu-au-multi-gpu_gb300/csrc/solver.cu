@@ -24,6 +24,7 @@
 #include "step_resident.cuh"
 #include "step_ring.cuh"
 #include "step_tma.cuh"
+#include "stream_sms.h"
 #include "forms.cuh"
 
 using namespace lbm_b200;
@@ -344,8 +345,13 @@ int launch_steps_o(lbm_solver* s, int steps) {
   }
 }
 
+// A cooperative launch that was refused because its blocks cannot all be resident: nothing of it
+// ran, and the step kernels take the steps.
+constexpr int kRefused = -1;
+
 // Resident launches: the whole run of `steps` in cooperative launches of at most
-// kResidentSteps steps each, the state in the blocks' shared memory meanwhile.
+// kResidentSteps steps each, the state in the blocks' shared memory meanwhile. kRefused with the
+// first of them.
 template <class ST, bool kOpen, int kForce>
 int launch_resident_t(lbm_solver* s, int steps) {
   using Phys = typename Form<ST>::Phys;
@@ -372,41 +378,46 @@ int launch_resident_t(lbm_solver* s, int steps) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  s->last_grid = s->res.tx * s->res.ty;
-  s->last_variant = kVariantResident;
-  while (steps > 0) {
-    const int n = std::min(steps, kResidentSteps);
-    LBM_CUDA(s, cudaLaunchKernelEx(&cfg, kernel, a, s->res, n, static_cast<LLWord*>(s->outbox), s->err_flag));
+  for (int done = 0; done < steps;) {
+    const int n = std::min(steps - done, kResidentSteps);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, s->res, n, static_cast<LLWord*>(s->outbox), s->err_flag);
+    if (e == cudaErrorCooperativeLaunchTooLarge && done == 0) {
+      cudaGetLastError();
+      return kRefused;
+    }
+    LBM_CUDA(s, e);
     LBM_CUDA(s, launch_dependent(counter_add_dep_kernel, dim3(1), dim3(1), 0, s->stream, s->step_ctr,
                                  static_cast<uint32_t>(n)));
-    steps -= n;
+    done += n;
   }
+  s->last_grid = s->res.tx * s->res.ty;
+  s->last_variant = kVariantResident;
   return LBM_OK;
 }
 
 template <class ST>
 int launch_resident(lbm_solver* s, int steps) {
-  int rc = LBM_OK;
-  with_force(Form<ST>::consts(s->tau, s->fx, s->fy).force, [&](auto kind) {
-    constexpr int K = decltype(kind)::value;
-    rc = s->open_x ? launch_resident_t<ST, true, K>(s, steps) : launch_resident_t<ST, false, K>(s, steps);
-  });
+  int rc = kRefused;
+  if constexpr (sizeof(ST) != 8)
+    with_force(Form<ST>::consts(s->tau, s->fx, s->fy).force, [&](auto kind) {
+      constexpr int K = decltype(kind)::value;
+      rc = s->open_x ? launch_resident_t<ST, true, K>(s, steps) : launch_resident_t<ST, false, K>(s, steps);
+    });
   return rc;
 }
 
 // Do the step kernels' launch sequences end with a counter update?
 bool counts_steps(const lbm_solver* s) { return s->elem == 2; }
 
-// Runs of at least kResidentMinSteps steps take resident launches where the grid fits and the
-// caller has not chosen a kernel.
+// Runs of at least kResidentMinSteps steps take resident launches where the grid fits, its blocks
+// the SMs that the stream may use, and the caller has not chosen a kernel.
 bool use_resident(const lbm_solver* s, int steps) {
-  return s->res.tx > 0 && s->variant < 0 && s->grid == 0 && s->block == kStepThreads && steps >= kResidentMinSteps;
+  return s->res.tx > 0 && s->variant < 0 && s->grid == 0 && s->block == kStepThreads && steps >= kResidentMinSteps &&
+         s->res.tx * s->res.ty <= stream_sm_count(s->stream, s->sm_count);
 }
 
 template <class ST>
 int launch_steps(lbm_solver* s, int steps) {
-  if constexpr (sizeof(ST) != 8)
-    if (use_resident(s, steps)) return launch_resident<ST>(s, steps);
   const int rc = s->open_x ? launch_steps_o<ST, true>(s, steps) : launch_steps_o<ST, false>(s, steps);
   if (rc) return rc;
   // The counter keys the rounding of the 16-bit forms (and numbers resident states, whose launches
@@ -569,6 +580,7 @@ PlaneScales default_scales(int precision) {
 namespace lbm_b200 {
 
 int solver_launch(lbm_solver* s, int steps) { LBM_DISPATCH(s, launch_steps, s, steps); }
+static int solver_launch_resident(lbm_solver* s, int steps) { LBM_DISPATCH(s, launch_resident, s, steps); }
 
 void drop_step_graph(lbm_solver* s) {
   if (s->graph) cudaGraphExecDestroy(s->graph);
@@ -610,10 +622,16 @@ int ensure_step_graph(lbm_solver* s) {
   return LBM_OK;
 }
 
-// Steps: whole CUDA graphs of kGraphSteps launches for long runs on a non-default stream (no
-// per-launch host overhead, which dominates small grids), direct launches for the remainder.
+// Steps: resident launches where they apply, else whole CUDA graphs of kGraphSteps launches for long
+// runs on a non-default stream (no per-launch host overhead, which dominates small grids), direct
+// launches for the remainder.
 int solver_step_raw(lbm_solver* s, int steps) {
-  if (s->graphs && s->stream != nullptr && steps >= kGraphSteps && !use_resident(s, steps)) {
+  if (use_resident(s, steps)) {
+    const int rc = solver_launch_resident(s, steps);
+    if (!rc) s->kernels += steps + 1;
+    if (rc != kRefused) return rc;
+  }
+  if (s->graphs && s->stream != nullptr && steps >= kGraphSteps) {
     if (int rc = ensure_step_graph(s)) return rc;
     while (s->graph && steps >= kGraphSteps) {
       LBM_CUDA(s, cudaGraphLaunch(s->graph, s->stream));
@@ -622,9 +640,8 @@ int solver_step_raw(lbm_solver* s, int steps) {
     }
   }
   if (steps <= 0) return LBM_OK;
-  const bool update = counts_steps(s) || use_resident(s, steps);
   const int rc = solver_launch(s, steps);
-  if (!rc) s->kernels += steps + (update ? 1 : 0);
+  if (!rc) s->kernels += steps + (counts_steps(s) ? 1 : 0);
   return rc;
 }
 
