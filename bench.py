@@ -636,7 +636,7 @@ def run_ours(args):
     barrier(dist)
     torch.cuda.synchronize()
     solver.synchronize()
-    k_before = solver.kernel_launches()
+    k_before = solver.enqueued_kernels()
     host = [time.perf_counter()]
     events[0].record(stream)
     for k, ev in zip(sizes, events[1:]):
@@ -646,7 +646,7 @@ def run_ours(args):
         ev.synchronize()
         host.append(time.perf_counter())
     solver.synchronize()
-    launches = solver.kernel_launches() - k_before
+    launches = solver.enqueued_kernels() - k_before
     torch.cuda.synchronize()
     barrier(dist)
     rep_secs = [events[k].elapsed_time(events[k + 1]) * 1e-3 for k in range(reps)]

@@ -114,11 +114,16 @@ int lbm_timed_run(lbm_solver* s, int steps, double* seconds);
 /* Waits for all work of s. */
 int lbm_synchronize(lbm_solver* s);
 
-/* Number of kernels s has enqueued for time steps so far: one per step, plus one step-counter
- * update per launch sequence of the 16-bit forms and per resident launch (a replayed step graph counts the kernels it holds, a launch that
- * takes many steps counts one per step). For
- * benchmarks that report how many of the library's kernels ran in a timed region. */
+/* The work of s's time steps so far, at one kernel per step: the steps taken, plus one step-counter
+ * update per launch sequence of the 16-bit forms (a replayed step graph is one) and per resident run.
+ * Steps that share a launch count one by one, so that the figure grows alike on every grid. */
 int lbm_kernel_launches(const lbm_solver* s, long long* count);
+
+/* Number of kernels that s has really enqueued for time steps so far: step kernels and step-counter
+ * updates, those of replayed graphs among them, and two (the launch and its update) for each
+ * resident launch of up to 8192 steps. For benchmarks that report how many of the library's kernels
+ * ran in a timed region. */
+int lbm_enqueued_kernels(const lbm_solver* s, long long* count);
 
 /* Replaces SolverV3::populations() (solver_v3.cu:300-320): post-streaming populations in v0
  * layout into s_host (nx*ny*9 values of the host type), solid cells 0. The gather runs on the

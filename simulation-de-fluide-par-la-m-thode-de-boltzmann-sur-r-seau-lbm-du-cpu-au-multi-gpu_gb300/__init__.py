@@ -94,6 +94,7 @@ def lib() -> C.CDLL:
             "lbm_adj_get_populations": ([vp, i, vp], i),
             "lbm_adj_step_times": ([vp, C.POINTER(d), C.POINTER(d)], i),
             "lbm_kernel_launches": ([vp, C.POINTER(C.c_longlong)], i),
+            "lbm_enqueued_kernels": ([vp, C.POINTER(C.c_longlong)], i),
             "lbm_adj_set_tiles": ([vp, i, i], i),
             "lbm_adj_get_tiles": ([vp, C.POINTER(i), C.POINTER(i)], i),
             "lbm_batch_create": ([i, vp, vp, vp, vp, vp, vp, i, C.POINTER(vp)], i),
@@ -242,9 +243,16 @@ class Solver:
         return 0
 
     def kernel_launches(self) -> int:
-        """Kernels enqueued for time steps so far (step launches and step-counter updates)."""
+        """Time steps so far at one kernel per step, and step-counter updates; steps that share a
+        launch count one by one (enqueued_kernels counts launches)."""
         n = C.c_longlong(0)
         self._check(lib().lbm_kernel_launches(self._h, C.byref(n)))
+        return n.value
+
+    def enqueued_kernels(self) -> int:
+        """Kernels really enqueued for time steps so far, those of replayed graphs among them."""
+        n = C.c_longlong(0)
+        self._check(lib().lbm_enqueued_kernels(self._h, C.byref(n)))
         return n.value
 
     def bench_info(self) -> str:

@@ -388,6 +388,7 @@ int launch_resident_t(lbm_solver* s, int steps) {
     LBM_CUDA(s, e);
     LBM_CUDA(s, launch_dependent(counter_add_dep_kernel, dim3(1), dim3(1), 0, s->stream, s->step_ctr,
                                  static_cast<uint32_t>(n)));
+    s->enqueued += 2;
     done += n;
   }
   s->last_grid = s->res.tx * s->res.ty;
@@ -636,12 +637,16 @@ int solver_step_raw(lbm_solver* s, int steps) {
     while (s->graph && steps >= kGraphSteps) {
       LBM_CUDA(s, cudaGraphLaunch(s->graph, s->stream));
       s->kernels += kGraphSteps + (counts_steps(s) ? 1 : 0);  // the graph's launches
+      s->enqueued += kGraphSteps + (counts_steps(s) ? 1 : 0);
       steps -= kGraphSteps;
     }
   }
   if (steps <= 0) return LBM_OK;
   const int rc = solver_launch(s, steps);
-  if (!rc) s->kernels += steps + (counts_steps(s) ? 1 : 0);
+  if (!rc) {
+    s->kernels += steps + (counts_steps(s) ? 1 : 0);
+    s->enqueued += steps + (counts_steps(s) ? 1 : 0);
+  }
   return rc;
 }
 
@@ -893,6 +898,12 @@ int lbm_run(lbm_solver* s, int steps) {
 int lbm_kernel_launches(const lbm_solver* s, long long* count) {
   if (!s || !count) return LBM_ERR_INVALID_ARG;
   *count = s->kernels;
+  return LBM_OK;
+}
+
+int lbm_enqueued_kernels(const lbm_solver* s, long long* count) {
+  if (!s || !count) return LBM_ERR_INVALID_ARG;
+  *count = s->enqueued;
   return LBM_OK;
 }
 
