@@ -194,11 +194,14 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks);
  * 28); 16-bit storage: 19 below 2^21 cells, 17 below 2^22 and on rows that fill 2048-cell tiles
  * badly, else 20 (from 2^23 cells on with 2 blocks per SM, 27); FP64: kernels of its own that
  * multiply on the integer units, bit for bit the same (25: a ring, 26: the direct kernel, for rows
- * below 256 cells or whose 256-cell tiles are less than 95 % full).
+ * below 256 cells or whose 256-cell tiles are less than 95 % full, with 128 threads per block unless
+ * lbm_set_launch gives a number).
  * With -1 and no launch shape set, runs of at least 4 steps of an FP32 or 16-bit grid that fits the
  * SMs' shared memory (up to about 370k cells in FP32, 750k with 16-bit storage, depending on the
  * shape) keep the state there for the whole call, in one cooperative launch (24); on a stream whose
  * SMs are fewer than its blocks (a green context) the step kernels take them.
+ * 23 to 28 can be set too, on a solver whose precision and grid they are for (24: as -1 does where
+ * its runs are long enough); others are refused.
  * The 16-bit forms round stored populations stochastically (see lbm_create); every variant
  * derives the same random bits, so the variants give the same results. */
 int lbm_set_variant(lbm_solver* s, int variant);

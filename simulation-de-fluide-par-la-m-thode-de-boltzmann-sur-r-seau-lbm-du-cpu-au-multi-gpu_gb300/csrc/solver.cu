@@ -90,7 +90,7 @@ int launch_steps_t(lbm_solver* s, int steps) {
   // FP64 with integer multiplications holds 141 registers: blocks of half the size let 12 warps
   // reside instead of 8 and even out the last wave (300 x 300: 2.60k MLUPS with 256 threads).
   constexpr bool kInt = std::is_same_v<Phys, F64IntPhys>;
-  const int block = kInt ? std::min(s->block, 128) : s->block;
+  const int block = kInt && !s->block_set ? 128 : s->block;
   int grid = s->grid;
   if (grid <= 0) {
     int per_sm = 0;
@@ -100,6 +100,7 @@ int launch_steps_t(lbm_solver* s, int steps) {
     const int need = (a.items + warps_per_block - 1) / warps_per_block;
     grid = std::max(1, std::min(need, std::max(1, per_sm) * s->sm_count));
   }
+  s->last_block = block;
   s->last_grid = grid;
   for (int k = 0; k < steps; ++k) {
     a.src = static_cast<const ST*>(s->buf[s->cur]);
@@ -243,7 +244,7 @@ int launch_ring_t(lbm_solver* s, int steps) {
   }
 }
 
-// Internal variant of the automatic choice: the ring with 4 consumer warps, 2 passes (256-cell
+// Variant of the automatic choice: the ring with 4 consumer warps, 2 passes (256-cell
 // tiles), 2 stages and 5 resident blocks per SM, for plain FP32 on large grids. With fewer
 // instructions per cell the earlier choice (12, then 63 registers and so 3 blocks) drains its
 // stages faster and keeps too many bytes queued: 4096^2 MLUPS by shape and blocks per SM: 12
@@ -254,15 +255,14 @@ int launch_ring_t(lbm_solver* s, int steps) {
 // 90.6k.
 constexpr int kVariantF32Large = 23, kVariantF32Largest = 28;
 
-// Internal variant of the automatic choice: 20 with at most 2 resident blocks per SM, for 16-bit
+// Variant of the automatic choice: 20 with at most 2 resident blocks per SM, for 16-bit
 // storage on grids of at least 2^23 cells.
 constexpr int kVariant16Large = 27;
 
-// Internal variants of the automatic choice in FP64: ring and direct kernel with integer
-// multiplications.
+// Variants of the automatic choice in FP64: ring and direct kernel with integer multiplications.
 constexpr int kVariantF64Ring = 25, kVariantF64Direct = 26;
 
-// Internal variant number of resident launches (step_resident.cuh). A launch loads and stores the
+// Variant number of resident launches (step_resident.cuh). A launch loads and stores the
 // state and has no dependent-launch overlap, so short runs stay with the step kernels (us a step,
 // resident against them, runs of 2 / 3 / 4 / 16 / 400 steps: FP32 128 x 66 6.5 / 5.3 / 3.6 / 1.9 /
 // 1.4 against 6.5 / 5.2 / 4.7 / 3.5 / 3.0; 1024 x 256 8.5 / 7.4 / 5.6 / 3.3 / 2.5 against 8.4 / 7.5 /
@@ -310,10 +310,17 @@ int auto_variant(const lbm_solver* s) {
 
 template <class ST, bool kOpen>
 int launch_steps_o(lbm_solver* s, int steps) {
-  s->last_variant = s->variant >= 0 ? s->variant : auto_variant<ST>(s);
+  s->last_variant = s->variant >= 0 && s->variant != kVariantResident ? s->variant : auto_variant<ST>(s);
+  s->last_block = 0;
+  // The automatic choice's own kernels, of one storage form each.
   if constexpr (sizeof(ST) == 8) {
     if (s->last_variant == kVariantF64Ring) return launch_ring_t<ST, kOpen, 8, 1, 4, 3, 0, F64IntPhys>(s, steps);
     if (s->last_variant == kVariantF64Direct) return launch_steps_t<ST, kOpen, 0, F64IntPhys>(s, steps);
+  } else if constexpr (sizeof(ST) == 4) {
+    if (s->last_variant == kVariantF32Large) return launch_ring_t<ST, kOpen, 4, 2, 2, 5, 5>(s, steps);
+    if (s->last_variant == kVariantF32Largest) return launch_ring_t<ST, kOpen, 4, 2, 3, 1, 3>(s, steps);
+  } else {
+    if (s->last_variant == kVariant16Large) return launch_ring_t<ST, kOpen, 8, 4, 2, 2, 2>(s, steps);
   }
   switch (s->last_variant) {
     case 1: return launch_steps_t<ST, kOpen, 1>(s, steps);
@@ -337,9 +344,6 @@ int launch_steps_o(lbm_solver* s, int steps) {
     case 19: return launch_ring_t<ST, kOpen, 8, 1, 4, 3>(s, steps);
     case 20: return launch_ring_t<ST, kOpen, 8, 4, 2, 2>(s, steps);
     case 21: return launch_ring_t<ST, kOpen, 4, 4, 2, 5>(s, steps);
-    case kVariant16Large: return launch_ring_t<ST, kOpen, 8, 4, 2, 2, sizeof(ST) == 2 ? 2 : 0>(s, steps);
-    case kVariantF32Large: return launch_ring_t<ST, kOpen, 4, 2, 2, 5, 5>(s, steps);
-    case kVariantF32Largest: return launch_ring_t<ST, kOpen, 4, 2, 3, 1, 3>(s, steps);
     case 22: return launch_ring_t<ST, kOpen, 8, 4, 3, 2>(s, steps);
     default: return launch_steps_t<ST, kOpen, 0>(s, steps);
   }
@@ -393,6 +397,7 @@ int launch_resident_t(lbm_solver* s, int steps) {
   }
   s->last_grid = s->res.tx * s->res.ty;
   s->last_variant = kVariantResident;
+  s->last_block = 0;
   return LBM_OK;
 }
 
@@ -413,7 +418,7 @@ bool counts_steps(const lbm_solver* s) { return s->elem == 2; }
 // Runs of at least kResidentMinSteps steps take resident launches where the grid fits, its blocks
 // the SMs that the stream may use, and the caller has not chosen a kernel.
 bool use_resident(const lbm_solver* s, int steps) {
-  return s->res.tx > 0 && s->variant < 0 && s->grid == 0 && s->block == kStepThreads && steps >= kResidentMinSteps &&
+  return s->res.tx > 0 && (s->variant < 0 || s->variant == kVariantResident) && s->grid == 0 && s->block == kStepThreads && steps >= kResidentMinSteps &&
          s->res.tx * s->res.ty <= stream_sm_count(s->stream, s->sm_count);
 }
 
@@ -1114,7 +1119,7 @@ int lbm_device_info(lbm_solver* s, char* buf, size_t size) {
       "\", \"cuda_runtime\": \"" + ver(runtime) + "\", \"cuda_compiled\": \"" +
       ver(CUDART_VERSION) + "\", \"ecc\": " + std::to_string(prop.ECCEnabled) +
       ", \"sm_count\": " + std::to_string(s->sm_count) + ", \"block\": \"" +
-      std::to_string(s->block) + "x1\", \"grid\": " + std::to_string(s->last_grid) +
+      std::to_string(s->last_block ? s->last_block : s->block) + "x1\", \"grid\": " + std::to_string(s->last_grid) +
       ", \"variant\": \"b200_pull_vec" + std::to_string(s->vec) +
       "_v" + std::to_string(s->last_variant) + (s->variant < 0 ? "_auto" : "") + "\", \"precision\": \"" +
       names[s->precision] + "\"";
@@ -1132,10 +1137,12 @@ int lbm_get_shape(const lbm_solver* s, int* nx, int* ny, int* precision) {
 
 int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks) {
   if (check(s)) return LBM_ERR_INVALID_ARG;
-  if (block_threads <= 0) block_threads = kStepThreads;
+  const bool given = block_threads > 0;
+  if (!given) block_threads = kStepThreads;
   if (block_threads % 32 != 0 || block_threads > kStepThreads || grid_blocks < 0)
     return set_error(s, LBM_ERR_INVALID_ARG, "block must be a multiple of 32 and <= 256");
   s->block = block_threads;
+  s->block_set = given;
   s->grid = grid_blocks;
   lbm_b200::drop_step_graph(s);
   return LBM_OK;
@@ -1143,8 +1150,14 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks) {
 
 int lbm_set_variant(lbm_solver* s, int variant) {
   if (check(s)) return LBM_ERR_INVALID_ARG;
-  if (variant < -1 || variant > 22)
-    return set_error(s, LBM_ERR_INVALID_ARG, "variant must be in [-1, 22]");
+  // 23 to 28 are of one storage form each; resident launches need a grid that fits.
+  bool ok = variant >= -1 && variant <= kVariantF32Largest;
+  if (variant == kVariantF32Large || variant == kVariantF32Largest) ok = s->elem == 4;
+  if (variant == kVariantResident) ok = s->res.tx > 0;
+  if (variant == kVariantF64Ring || variant == kVariantF64Direct) ok = s->elem == 8;
+  if (variant == kVariant16Large) ok = s->elem == 2;
+  if (!ok)
+    return set_error(s, LBM_ERR_INVALID_ARG, "variant must be in [-1, 22], or a larger one of the solver's precision and grid");
   s->variant = variant;
   lbm_b200::drop_step_graph(s);
   return LBM_OK;

@@ -47,7 +47,10 @@ struct lbm_solver {
   int red_blocks = 0;
   void* stage = nullptr;  // device staging for host input / output
   size_t stage_bytes = 0;
-  int block = 256, grid = 0, last_grid = 0;  // step launch shape (grid 0: persistent, automatic)
+  // Step launch shape (grid 0: persistent, automatic; block_set: the caller chose the block size).
+  int block = 256, grid = 0, last_grid = 0;
+  bool block_set = false;
+  int last_block = 0;  // threads of the last direct launch where they are not `block`
   // Set by a step kernel whose bounded wait ran out: in `box` where kernels reach host memory
   // (direct), else in device memory.
   int* err_flag = nullptr;
