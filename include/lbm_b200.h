@@ -211,13 +211,14 @@ int lbm_set_variant(lbm_solver* s, int variant);
 int lbm_state_view(lbm_solver* s, void** current, long long* plane_stride, int* row_pitch);
 
 /* Test setting, no counterpart in the reference: the limit, in non-blocking polls, of a ring
- * step kernel's first wait for a staged tile (variants 12-22 of lbm_step / lbm_run, on the
- * current device, for every solver). 0 restores the default (the ordinary bounded wait). A
- * small limit makes that wait run out on purpose, so that the failure path can be tested
- * without a wait that never ends: the kernel sets its error flag, lets every copy it issued
- * land and finishes without computing the rest of its tiles, and the next synchronising call
- * (lbm_run, lbm_synchronize, ...) returns LBM_ERR_TIMEOUT and clears the flag. The state is
- * then invalid until it is set again. */
+ * step kernel's first wait for a staged tile (variants 12-23, 25, 27 and 28 of lbm_step / lbm_run, on
+ * the current device, for every solver), and of each wait of a resident launch's block for its
+ * neighbours (solvers and ensembles, launches enqueued later). 0 restores the default (the
+ * ordinary bounded waits). A small limit makes such a wait run out on purpose, so that the failure
+ * path can be tested without a wait that never ends: the kernel sets its error flag, lets every copy
+ * it issued land and finishes without computing the rest of its tiles or steps, and the next
+ * synchronising call (lbm_run, lbm_synchronize, ...) returns LBM_ERR_TIMEOUT and clears the flag.
+ * The state is then invalid until it is set again. */
 int lbm_test_set_consumer_wait_limit(unsigned polls);
 
 /* ---------------------------------------------------------------------------------------------

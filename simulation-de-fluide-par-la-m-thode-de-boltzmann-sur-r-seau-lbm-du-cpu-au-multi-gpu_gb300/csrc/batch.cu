@@ -417,7 +417,7 @@ struct ResInst {
 template <class ST, class Phys, int kForce>
 __global__ void __launch_bounds__(res_threads<ST>(), 1)
     batch_resident_kernel(const StagedArgs<ST, Phys>* args, int parity, const ResBlock* blocks, const ResInst* insts,
-                          int steps, LLWord* outboxes, const uint32_t* tag_ctr, int* err) {
+                          int steps, LLWord* outboxes, const uint32_t* tag_ctr, int* err, unsigned polls_limit) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ StagedArgs<ST, Phys> s_args;
   __shared__ ResInst s_inst;
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(res_threads<ST>(), 1)
   if (threadIdx.x == 0) s_inst = insts[b.inst];
   __syncthreads();
   resident_body<ST, Phys, false, kForce>(smem, s_args.p, s_inst.L, b.tile, steps, outboxes + s_inst.out_off, tag_ctr,
-                                         err);
+                                         err, polls_limit);
 }
 static_assert(kResSmemBytes + 1024 <= 227 * 1024, "the resident block's arguments fit beside its buffers");
 
@@ -896,7 +896,8 @@ int launch_resident_k(lbm_batch* b, int steps) {
                            reinterpret_cast<const ResBlock*>(reinterpret_cast<char*>(b->mask_d) + b->res_block_at),
                            reinterpret_cast<const ResInst*>(reinterpret_cast<char*>(b->mask_d) + b->res_inst_at), n,
                            reinterpret_cast<LLWord*>(static_cast<char*>(b->buf[1]) + b->res_out_at),
-                           static_cast<const uint32_t*>(b->step_d + 2), reinterpret_cast<int*>(b->step_d + 1));
+                           static_cast<const uint32_t*>(b->step_d + 2), reinterpret_cast<int*>(b->step_d + 1),
+                           g_resident_polls.load());
     if (e == cudaErrorCooperativeLaunchTooLarge && done == 0) {
       cudaGetLastError();
       return kRefused;
@@ -1174,7 +1175,7 @@ int check_batch_flag(lbm_batch* b) {
   B_CUDA(b, cudaStreamSynchronize(b->stream));
   if (flag) {
     B_CUDA(b, cudaMemsetAsync(b->step_d + 1, 0, sizeof(flag), b->stream));
-    return bfail(b, LBM_ERR_TIMEOUT, "a step kernel gave up waiting for its shared-memory ring");
+    return bfail(b, LBM_ERR_TIMEOUT, kWaitMessage);
   }
   return LBM_OK;
 }

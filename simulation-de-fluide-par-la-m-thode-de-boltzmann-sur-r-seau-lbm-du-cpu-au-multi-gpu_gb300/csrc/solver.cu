@@ -384,7 +384,8 @@ int launch_resident_t(lbm_solver* s, int steps) {
   cfg.numAttrs = 1;
   for (int done = 0; done < steps;) {
     const int n = std::min(steps - done, kResidentSteps);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, s->res, n, static_cast<LLWord*>(s->outbox), s->err_flag);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, s->res, n, static_cast<LLWord*>(s->outbox), s->err_flag,
+                                             g_resident_polls.load());
     if (e == cudaErrorCooperativeLaunchTooLarge && done == 0) {
       cudaGetLastError();
       return kRefused;
@@ -584,6 +585,8 @@ PlaneScales default_scales(int precision) {
 // Internal helpers shared with the other translation units
 // ----------------------------------------------------------------------------------------------
 namespace lbm_b200 {
+
+std::atomic<unsigned> g_resident_polls{kResidentPolls};
 
 int solver_launch(lbm_solver* s, int steps) { LBM_DISPATCH(s, launch_steps, s, steps); }
 static int solver_launch_resident(lbm_solver* s, int steps) { LBM_DISPATCH(s, launch_resident, s, steps); }
@@ -877,7 +880,7 @@ static int check_step_flag(lbm_solver* s) {
     LBM_CUDA(s, cudaStreamSynchronize(s->stream));
     if (!s->box.flag) return LBM_OK;
     s->box.flag = 0;
-    return set_error(s, LBM_ERR_TIMEOUT, "a step kernel gave up waiting for its shared-memory ring");
+    return set_error(s, LBM_ERR_TIMEOUT, kWaitMessage);
   }
   int flag = 0;
   LBM_CUDA(s, cudaMemcpyAsync(&flag, s->err_flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
@@ -885,7 +888,7 @@ static int check_step_flag(lbm_solver* s) {
   if (flag) {
     LBM_CUDA(s, cudaMemsetAsync(s->err_flag, 0, sizeof(int), s->stream));
     LBM_CUDA(s, cudaStreamSynchronize(s->stream));
-    return set_error(s, LBM_ERR_TIMEOUT, "a step kernel gave up waiting for its shared-memory ring");
+    return set_error(s, LBM_ERR_TIMEOUT, kWaitMessage);
   }
   return LBM_OK;
 }
@@ -1173,6 +1176,7 @@ int lbm_state_view(lbm_solver* s, void** current, long long* plane_stride, int* 
 
 int lbm_test_set_consumer_wait_limit(unsigned polls) {
   const unsigned v = polls == 0 || polls >= lbm_b200::kSpinLimit ? lbm_b200::kSpinLimit : polls;
+  lbm_b200::g_resident_polls = std::min(v, lbm_b200::kResidentPolls);
   const cudaError_t e = cudaMemcpyToSymbol(lbm_b200::c_consumer_wait_limit, &v, sizeof v);
   return e == cudaSuccess ? LBM_OK : LBM_ERR_CUDA;
 }

@@ -3,12 +3,21 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
 
 #include "lbm_device.cuh"
 #include "resident_layout.h"
+
+namespace lbm_b200 {
+// Message of LBM_ERR_TIMEOUT.
+constexpr char kWaitMessage[] =
+    "a step kernel gave up waiting (for its shared-memory ring, or a resident launch's block for its neighbours)";
+// Looks at a word that a resident launch's block waits for: kResidentPolls, less only in tests.
+extern std::atomic<unsigned> g_resident_polls;
+}  // namespace lbm_b200
 
 // Results that kernels write straight into host memory (where the device can).
 struct alignas(64) HostBox {

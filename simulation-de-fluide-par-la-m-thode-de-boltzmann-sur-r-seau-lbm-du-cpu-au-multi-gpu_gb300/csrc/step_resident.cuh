@@ -33,8 +33,9 @@
 //     of the tile is done (512^2 3.16 against 2.47 us); two FP32 cells per lane in packed
 //     instructions (27 % fewer instructions, but 92 registers leave 20 warps for 29 items:
 //     1024 x 256 2.66 us, 512^2 2.70 us).
-//   * Waits are bounded (kResidentPolls); a wait that runs out sets the error flag and ends the
-//     block, and its neighbours' waits run out in turn.
+//   * Waits are bounded (kResidentPolls; a kernel argument, so that a test can shorten them); a wait
+//     that runs out sets the error flag and ends the block, and its neighbours' waits run out in
+//     turn.
 #pragma once
 
 #include "resident_layout.h"
@@ -236,11 +237,12 @@ __host__ __device__ constexpr int res_threads() {
 
 // The steps of tile `tile` of the grid p, cut as L. The state is read from and written back to
 // p.dst (p.src is unused); `outboxes` are the grid's, of both parities; *tag_ctr numbers the states
-// (it only ever grows, see above), *p.step_ctr keys the stochastic rounding.
+// (it only ever grows, see above), *p.step_ctr keys the stochastic rounding. A word is looked at
+// `polls_limit` times at most.
 template <class ST, class Phys, bool kOpen, int kForce>
 __device__ __forceinline__ void resident_body(unsigned char* smem, const StepArgs<ST, Phys>& p, const ResLayout& L,
                                               int tile, int steps, LLWord* outboxes, const uint32_t* tag_ctr,
-                                              int* err) {
+                                              int* err, unsigned polls_limit) {
   constexpr int PS = kResPlaneBytes / static_cast<int>(sizeof(ST));
   constexpr int LC = sizeof(ST) == 2 ? 2 : 1, kThreads = res_threads<ST>();
   ST* buf0 = reinterpret_cast<ST*>(smem);
@@ -323,8 +325,8 @@ __device__ __forceinline__ void resident_body(unsigned char* smem, const StepArg
     for (int e = kThreads - 1 - tid; e < npolls; e += kThreads) {
       const PollEntry q = polls[e];
       LLWord v = ll_load(from + q.src);
-      for (unsigned n = 0; v.tag != tag; ++n) {
-        if (n >= kResidentPolls) {
+      for (unsigned n = 1; v.tag != tag; ++n) {
+        if (n >= polls_limit) {
           atomicExch(err, 1);
           ok = false;
           break;
@@ -386,9 +388,11 @@ __device__ __forceinline__ void resident_body(unsigned char* smem, const StepArg
 // One grid: block k has tile k.
 template <class ST, class Phys, bool kOpen, int kForce>
 __global__ void __launch_bounds__(res_threads<ST>(), 1)
-    resident_step_kernel(const StepArgs<ST, Phys> p, const ResLayout L, int steps, LLWord* outboxes, int* err) {
+    resident_step_kernel(const StepArgs<ST, Phys> p, const ResLayout L, int steps, LLWord* outboxes, int* err,
+                         unsigned polls_limit) {
   extern __shared__ __align__(128) unsigned char smem[];
-  resident_body<ST, Phys, kOpen, kForce>(smem, p, L, static_cast<int>(blockIdx.x), steps, outboxes, p.step_ctr, err);
+  resident_body<ST, Phys, kOpen, kForce>(smem, p, L, static_cast<int>(blockIdx.x), steps, outboxes, p.step_ctr, err,
+                                         polls_limit);
 }
 
 }  // namespace lbm_b200
