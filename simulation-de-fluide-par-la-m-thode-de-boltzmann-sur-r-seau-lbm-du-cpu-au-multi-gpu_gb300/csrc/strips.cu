@@ -436,43 +436,44 @@ int set_t(lbm_strips* h, const void* s_host, Eq9<typename StoreTraits<ST>::T> eq
 }
 
 // Owned rows of every strip: v0-layout populations (what = 0) or rho/ux/uy (what = 1). The gather
-// kernels write each strip's owned rows where they lie in the whole lattice: in the host output
-// itself where kernels can address it, else in device memory that is copied once.
+// kernels write each strip's owned rows where they lie in the whole lattice, in the host output
+// itself, where kernels can address it; else strip after strip goes through a staging buffer of
+// one strip (a lattice may fill the device but for that).
 template <class ST>
 int get_t(lbm_strips* h, int what, void* out0, void* out1, void* out2) {
   using T = typename StoreTraits<ST>::T;
   using A = typename Form<ST>::A;
-  const int nx = h->nx, fields = what == 0 ? 1 : 3;
-  const size_t n = static_cast<size_t>(nx) * h->ny, bytes = n * (what == 0 ? kQ : 1) * sizeof(T);
+  const int nx = h->nx, fields = what == 0 ? 1 : 3, per_cell = what == 0 ? kQ : 1;
+  const size_t row_bytes = static_cast<size_t>(nx) * per_cell * sizeof(T);
   const Eq9<T> eq_in = strip_inlet<ST>(h, false);
   void* outs[3] = {out0, out1, out2};
-  T* dst[3] = {nullptr, nullptr, nullptr};
+  char* whole[3] = {nullptr, nullptr, nullptr};
   bool in_place = true;
   for (int f = 0; f < fields && in_place; ++f) {
-    dst[f] = static_cast<T*>(host_view(outs[f], bytes, sizeof(T), h->direct, true));
-    in_place = dst[f] != nullptr;
-  }
-  if (!in_place) {
-    if (int rc = ensure_stage(h, fields * bytes)) return rc;
-    for (int f = 0; f < fields; ++f) dst[f] = reinterpret_cast<T*>(static_cast<char*>(h->stage) + f * bytes);
-  }
-  for (int k = 0; k < h->strips; ++k) {
-    const Grid2D g = strip_grid(h, k);
-    const size_t at = static_cast<size_t>(h->y0[k]) * nx;
-    const ST* R = static_cast<const ST*>(h->buf[h->cur]) + h->off[k];
-    const int grid = grid_cells(h, static_cast<long long>(nx) * h->n[k]);
-    if (what == 0)
-      get_state_kernel<ST><<<grid, kGetThreads, 0, h->stream>>>(R, h->mask_d + h->moff[k], g, eq_in, h->sc, dst[0] + at * kQ,
-                                                        1, h->n[k]);
-    else
-      moments_kernel<ST, A><<<grid, 256, 0, h->stream>>>(R, h->mask_d + h->moff[k], g, eq_in, h->sc,
-                                                         T(T(0.5) * T(h->fx)), T(T(0.5) * T(h->fy)), dst[0] + at,
-                                                         dst[1] + at, dst[2] + at, 1, h->n[k]);
-    S_CUDA(h, cudaGetLastError());
+    whole[f] = static_cast<char*>(host_view(outs[f], row_bytes * h->ny, sizeof(T), h->direct, true));
+    in_place = whole[f] != nullptr;
   }
   if (!in_place)
+    if (int rc = ensure_stage(h, fields * row_bytes * *std::max_element(h->n.begin(), h->n.end()))) return rc;
+  for (int k = 0; k < h->strips; ++k) {
+    const Grid2D g = strip_grid(h, k);
+    const size_t at = row_bytes * h->y0[k], bytes = row_bytes * h->n[k];
+    const ST* R = static_cast<const ST*>(h->buf[h->cur]) + h->off[k];
+    const int grid = grid_cells(h, static_cast<long long>(nx) * h->n[k]);
+    T* dst[3] = {};
     for (int f = 0; f < fields; ++f)
-      S_CUDA(h, cudaMemcpyAsync(outs[f], dst[f], bytes, cudaMemcpyDeviceToHost, h->stream));
+      dst[f] = reinterpret_cast<T*>(in_place ? whole[f] + at : static_cast<char*>(h->stage) + f * bytes);
+    if (what == 0)
+      get_state_kernel<ST><<<grid, kGetThreads, 0, h->stream>>>(R, h->mask_d + h->moff[k], g, eq_in, h->sc, dst[0], 1,
+                                                                h->n[k]);
+    else
+      moments_kernel<ST, A><<<grid, 256, 0, h->stream>>>(R, h->mask_d + h->moff[k], g, eq_in, h->sc,
+                                                         T(T(0.5) * T(h->fx)), T(T(0.5) * T(h->fy)), dst[0], dst[1],
+                                                         dst[2], 1, h->n[k]);
+    S_CUDA(h, cudaGetLastError());
+    for (int f = 0; f < fields && !in_place; ++f)  // (the next strip's kernel waits for the copies)
+      S_CUDA(h, cudaMemcpyAsync(static_cast<char*>(outs[f]) + at, dst[f], bytes, cudaMemcpyDeviceToHost, h->stream));
+  }
   S_CUDA(h, cudaStreamSynchronize(h->stream));
   return LBM_OK;
 }
