@@ -200,6 +200,10 @@ int lbm_set_launch(lbm_solver* s, int block_threads, int grid_blocks);
  * SMs' shared memory (up to about 370k cells in FP32, 750k with 16-bit storage, depending on the
  * shape) keep the state there for the whole call, in one cooperative launch (24); on a stream whose
  * SMs are fewer than its blocks (a green context) the step kernels take them.
+ * Such a launch takes most SMs, so solvers that run at the same time on one GPU take turns (closed
+ * grids of at most 128 columns share the SMs). From about four such solvers of 10^4 to 10^5 cells on
+ * the step kernels, which overlap, are faster together: choose one (19, 17), or use an ensemble
+ * (lbm_batch), whose instances share one launch.
  * 23 to 28 can be set too, on a solver whose precision and grid they are for (24: as -1 does where
  * its runs are long enough); others are refused.
  * The 16-bit forms round stored populations stochastically (see lbm_create); every variant

@@ -203,10 +203,24 @@ inline int resident_items(const ResLayout& L) {
 }
 
 // Cuts an nx x ny grid into at most `blocks` tiles for kElem-byte storage: the fewest rounds of
-// the block's `warps` warps over its items, then the fewest items, then the shortest edge.
+// the block's `warps` warps over its items, then the fewest items, then the shortest edge. Closed
+// grids of at most 128 columns are cut into bands of one or two whole rows instead, 3/5 as many as
+// rows, where that is at most half the blocks: as fast for one solver (us a step, spread over the
+// SMs against bands: FP32 53 x 31 1.29 / 1.28, 64 x 64 1.29 / 1.29, 128 x 66 1.31 / 1.31, 120 x 40
+// 1.33 / 1.26, 75 x 81 1.31 / 1.39; FP16 128 x 66 1.49 / 1.47, 40 x 60 1.50 / 1.53), and it leaves
+// SMs to other solvers, whose resident launches otherwise wait (eight at once, us a step of all,
+// spread / bands / one launch per step: FP32 53 x 31 5.2 / 1.4 / 3.6, 128 x 66 10.6 / 3.6 / 3.8; FP16
+// 128 x 66 12.0 / 4.0 / 5.0). Bands cost more for one solver with wider rows (FP16 256 x 120 1.50 /
+// 1.58) and open ends (FP32 128 x 66 1.35 / 1.42), which stay spread, as do grids that need the SMs
+// (256 x 256: one solver 1.64 us on 152 SMs, 2.08 on 76; eight 12.9 / 8.4, one launch per step 9.4).
 // Returns a layout with tx = 0 when no cut fits.
 template <int kElem>
 inline ResLayout resident_layout(int nx, int ny, int blocks, int warps, bool open_x) {
+  const int bands = static_cast<int>((3LL * ny + 4) / 5);
+  if (!open_x && nx <= 128 && 2 * bands <= blocks) {
+    const ResLayout L = resident_cut<kElem>(nx, ny, 1, bands, false);
+    if (L.tx) return L;
+  }
   ResLayout best;
   long long best_cost = -1;
   for (int tx = 1; tx <= blocks; ++tx) {
