@@ -264,11 +264,10 @@ constexpr int kVariantF64Ring = 25, kVariantF64Direct = 26;
 
 // Variant number of resident launches (step_resident.cuh). A launch loads and stores the
 // state and has no dependent-launch overlap, so short runs stay with the step kernels (us a step,
-// resident against them, runs of 2 / 3 / 4 / 16 / 400 steps: FP32 128 x 66 6.5 / 5.3 / 3.6 / 1.9 /
-// 1.4 against 6.5 / 5.2 / 4.7 / 3.5 / 3.0; 1024 x 256 8.5 / 7.4 / 5.6 / 3.3 / 2.5 against 8.4 / 7.5 /
-// 7.2 / 5.6 / 5.1; FP16 1021 x 700 11.2 / 10.4 / 7.6 / 4.9 / 4.0 against 11.1 / 9.9 / 10.0 / 8.7 /
-// 8.3; below four steps both columns are the step kernels): from four steps on every size that
-// fits is faster resident.
+// resident against them, runs of 4 / 16 / 400 steps: FP32 128 x 66 3.2 / 1.8 / 1.3 against 3.6 /
+// 3.0 / 2.9; 1024 x 256 5.3 / 3.0 / 2.3 against 6.0 / 5.2 / 4.8; FP16 1021 x 700 7.0 / 4.3 / 3.4
+// against 8.9 / 8.2 / 7.9): from four steps on every size that fits is faster resident, for one
+// solver at a time (resident_layout.h has several).
 constexpr int kVariantResident = 24;
 
 // Automatic kernel choice (variant < 0), from a sweep of every variant on one GB300 (channel,

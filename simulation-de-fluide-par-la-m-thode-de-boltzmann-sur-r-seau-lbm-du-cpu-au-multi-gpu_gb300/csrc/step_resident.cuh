@@ -24,10 +24,10 @@
 //     barrier per step.
 //   * Bound by: instruction issue on the larger tiles (FP32 1024 x 256: 2.5 us a step, 57 items of
 //     about 270 instructions on 32 warps, 80 % issue between the barriers), the exchange's
-//     latency (about 0.9 us) on small ones (128 x 66: 1.4 us). us a step at 50 to 400 steps a call,
-//     with one launch per step in parentheses: FP32 53 x 31 1.4 (2.8), 256^2 1.7 (3.2), 512^2 2.5
-//     (5.3), 1024 x 256 2.5 (5.1), 1000 x 320 open 2.8 (6.3); FP16 128 x 66 1.6 (4.4), 512^2 2.5
-//     (4.3), 1021 x 700 4.0 (8.3).
+//     latency (about 0.9 us) on small ones (128 x 66: 1.3 us). us a step at 400 steps a call, with one
+//     launch per step in parentheses: FP32 53 x 31 1.3 (2.7), 256^2 1.7 (3.1), 512^2 2.3 (4.9), 1024
+//     x 256 2.4 (4.8), 1000 x 320 open 2.9 (6.6); FP16 128 x 66 1.5 (3.7), 512^2 2.4 (4.2), 1021 x 700
+//     3.4 (7.9).
 //   * Measured and left out: words of one value and an 8-byte tag (three times the stores and
 //     polls: 1024 x 256 2.90 us); whole-row items for the frame, which hold up the words until most
 //     of the tile is done (512^2 3.16 against 2.47 us); two FP32 cells per lane in packed
