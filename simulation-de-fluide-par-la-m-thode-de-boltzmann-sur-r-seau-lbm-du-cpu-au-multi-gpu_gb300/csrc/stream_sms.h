@@ -15,18 +15,17 @@ struct Driver {
   CUresult (*stream_green)(CUstream, CUgreenCtx*) = nullptr;
   CUresult (*green_resource)(CUgreenCtx, CUdevResource*, CUdevResourceType) = nullptr;
   Driver() {
-    auto find = [](const char* name, void* fn) {
+    auto find = [](const char* name) {
       cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
       void* p = nullptr;
-      if (cudaGetDriverEntryPointByVersion(name, &p, 13000, cudaEnableDefault, &q) != cudaSuccess ||
-          q != cudaDriverEntryPointSuccess) {
-        cudaGetLastError();
-        p = nullptr;
-      }
-      *static_cast<void**>(fn) = p;
+      if (cudaGetDriverEntryPointByVersion(name, &p, 13000, cudaEnableDefault, &q) == cudaSuccess &&
+          q == cudaDriverEntryPointSuccess)
+        return p;
+      cudaGetLastError();
+      return static_cast<void*>(nullptr);
     };
-    find("cuStreamGetGreenCtx", &stream_green);
-    find("cuGreenCtxGetDevResource", &green_resource);
+    stream_green = reinterpret_cast<decltype(stream_green)>(find("cuStreamGetGreenCtx"));
+    green_resource = reinterpret_cast<decltype(green_resource)>(find("cuGreenCtxGetDevResource"));
   }
 };
 }  // namespace stream_sms_detail
