@@ -1404,6 +1404,7 @@ int lbm_adj_set_alpha(lbm_adjoint* a, const double* alpha) {
   if (!alpha) {
     cudaFree(a->alpha);
     a->alpha = nullptr;
+    a->seg_last = false;  // a backward run computes its states without the field
     return LBM_OK;
   }
   const size_t n = static_cast<size_t>(a->batch) * a->g.nx * a->g.ny;
