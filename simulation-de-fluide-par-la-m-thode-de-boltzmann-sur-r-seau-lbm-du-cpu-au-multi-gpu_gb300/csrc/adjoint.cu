@@ -1086,6 +1086,7 @@ int forward_t(lbm_adjoint* a, const void* s0_host, int steps, int window, double
   const size_t sb = state_bytes(a);
   const size_t nckpt = static_cast<size_t>(steps / a->K) + 1;
   if (a->ckpt_count < nckpt) {
+    a->have_forward = false;  // an earlier run's checkpoints and final state go
     cudaFree(a->ckpt);
     a->ckpt = nullptr;
     a->ckpt_count = 0;
