@@ -8,7 +8,8 @@
 // kernel may not read or write at all is a fault that ends the CUDA context, where a copy would have
 // met an ordinary error of the host. So the pages of a pageable buffer are populated, for reading or
 // for writing, before it is used in place, also those that are there: that is what asks the host
-// whether they may be (pages of 64 KB that are there: 28 us for 77 MB).
+// whether they may be (pages of 64 KB that are there: 28 us for 77 MB in a row of such calls; a read
+// back of 4 MB takes 98 us with it, 93 us without).
 #pragma once
 
 #include <cuda_runtime.h>
